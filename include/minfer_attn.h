@@ -138,6 +138,16 @@ int minfer_attn_prefill(const MinferAttnPrefillParams* params, void* stream);
 size_t minfer_attn_prefill_workspace_bytes(int32_t batch, int32_t seq_q, int32_t seq_k);
 
 /*
+ * The larger scratch of a dense-mask call: the bytes above (rounded up to 16) plus
+ * 2 KB per mask tile, in which the classifying pass leaves the mixed tiles as one
+ * bit per (query, key).  The attention kernel then reads 16 bytes per row and mixed
+ * tile instead of the mask's 128, and masks whose rows are not 16-byte aligned
+ * (seq_k no multiple of 16) cost no more than aligned ones.  A workspace of at least
+ * this size is used that way; a smaller one as described above.
+ */
+size_t minfer_attn_prefill_workspace_bytes_bits(int32_t batch, int32_t seq_q, int32_t seq_k);
+
+/*
  * Decode attention over a padded KV cache (one query token per sequence).
  * No counterpart exists in the reference: its op insists on seq_q == seq_k
  * (op.cuh:76).  The cache layout is the one the reference's model skeleton

@@ -241,9 +241,14 @@ int minfer_attn_prefill(const MinferAttnPrefillParams* p, void* stream) {
     const size_t need = minfer_attn_prefill_workspace_bytes(p->batch, p->seq_q, p->seq_k);
     if (a.counter != nullptr && p->workspace_bytes >= need) {
       uint8_t* cls = static_cast<uint8_t*>(p->workspace) + 16;
-      cudaError_t ce = launch_mask_classify(a.mask, cls, p->batch, p->seq_q, p->seq_k, static_cast<cudaStream_t>(stream));
+      // the tiles' bits follow at the next 16-byte boundary when the caller's buffer has the room for them
+      uint32_t* bits = nullptr;
+      if (p->workspace_bytes >= minfer_attn_prefill_workspace_bytes_bits(p->batch, p->seq_q, p->seq_k))
+        bits = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(p->workspace) + ((need + 15) & ~static_cast<size_t>(15)));
+      cudaError_t ce = launch_mask_classify(a.mask, cls, bits, p->batch, p->seq_q, p->seq_k, static_cast<cudaStream_t>(stream));
       if (ce != cudaSuccess) return cuda_result(ce);
       a.cls = cls;
+      a.bits = bits;
     }
   }
   a.status = p->status;
@@ -268,6 +273,12 @@ size_t minfer_attn_prefill_workspace_bytes(int32_t batch, int32_t seq_q, int32_t
   if (batch <= 0 || seq_q <= 0 || seq_k <= 0) return 0;
   const size_t cls = static_cast<size_t>(batch) * ((seq_q + 127) / 128) * ((seq_k + 127) / 128);
   return 16 + cls;  // the work-item counter, then the tile classes of a dense mask
+}
+
+size_t minfer_attn_prefill_workspace_bytes_bits(int32_t batch, int32_t seq_q, int32_t seq_k) {
+  const size_t need = minfer_attn_prefill_workspace_bytes(batch, seq_q, seq_k);
+  if (need == 0) return 0;
+  return ((need + 15) & ~static_cast<size_t>(15)) + (need - 16) * (128 * 128 / 8);
 }
 
 int minfer_attn_rope_append(const MinferRopeParams* p, void* stream) {

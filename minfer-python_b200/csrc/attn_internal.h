@@ -22,6 +22,7 @@ struct PrefillArgs {
   void* out;
   const uint8_t* mask;
   const uint8_t* cls;     // per (batch, query tile, key tile) mask class, or null: see mask_classify.cu
+  const uint32_t* bits;   // per tile of cls 128 rows of 128 bits (valid for mixed tiles), or null: mask bytes are read
   int32_t* status;
   int* counter;           // persistent kernel: work-item counter in the caller's workspace, or null (static order)
   int64_t out_stride[3];  // elements: batch, head, row
@@ -53,8 +54,9 @@ cudaError_t launch_prefill_persist(const CUtensorMap& tq, const CUtensorMap& tk,
                                    bool bf16, cudaStream_t stream);
 
 // Classifies every 128 x 128 tile of a dense [batch, 1, seq_q, seq_k] byte mask: 0 = no byte set,
-// 1 = every in-range byte set, 2 = mixed.  cls is [batch, ceil(seq_q/128), ceil(seq_k/128)].
-cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, int batch, int seq_q, int seq_k,
+// 1 = every in-range byte set, 2 = mixed.  cls is [batch, ceil(seq_q/128), ceil(seq_k/128)]; bits (or null): per tile
+// of cls, 128 rows of 128 bits, written for mixed tiles only.
+cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, uint32_t* bits, int batch, int seq_q, int seq_k,
                                  cudaStream_t stream);
 
 // Kernel-side view of a RoPE + KV-append call.  Strides in elements.

@@ -8,6 +8,7 @@
 // structure at the cost of reading the mask once (HBM-bound, ~1 byte per
 // score instead of the B*H re-reads a per-head kernel would do).
 #include "attn_internal.h"
+#include "ptx.cuh"
 
 namespace minfer_attn {
 
@@ -15,54 +16,100 @@ namespace {
 
 constexpr int kTile = 128;
 
-// grid (key tiles, query tiles, batch), 256 threads: thread t handles row t/2,
-// 64 columns (half a tile row)
-__global__ void __launch_bounds__(256) mask_classify_kernel(const uint8_t* __restrict__ mask, uint8_t* __restrict__ cls,
-                                                            int seq_q, int seq_k) {
+// 16 columns of one mask row as words.
+__device__ __forceinline__ void row_words16(const uint8_t* __restrict__ p, uint32_t (&w)[4]) {
+  const uint32_t mis = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)) & 15u;
+  if (mis == 0) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+  } else {
+    // rows of a mask whose length is no multiple of 16 start anywhere: aligned words, shifted into place (every
+    // word read holds at least one byte of these 16 columns)
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - (mis & 3u));
+    const uint32_t sh = (mis & 3u) * 8u;
+    uint32_t a[5];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = __ldg(q + i);
+    a[4] = sh ? __ldg(q + 4) : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(a[i], a[i + 1], sh);
+  }
+}
+
+// grid (key tiles, query tiles, batch), 256 threads: 8 threads per row (16 columns each), 32 rows per pass, four
+// passes whose loads are all in flight together.  The class of a tile needs no bits: an OR of its words, and an AND of
+// their bytes' top bits after a carry (nonzero_bits below); computing every tile's bits first made the kernel
+// instruction-bound.  Mixed tiles then leave their bits behind (128 rows of 16 bytes), so that the attention
+// kernel, which needs a mixed tile once per head pair, reads 16 bytes per row instead of 128 and no row of it is
+// misaligned.
+__global__ void __launch_bounds__(256, 6) mask_classify_kernel(const uint8_t* __restrict__ mask, uint8_t* __restrict__ cls,
+                                                            uint32_t* __restrict__ bits, int seq_q, int seq_k) {
   const int kt = blockIdx.x, qt = blockIdx.y, b = blockIdx.z;
-  const int row = qt * kTile + (threadIdx.x >> 1);
-  const int col0 = kt * kTile + (threadIdx.x & 1) * 64;
-  bool any = false, all = true;
-  if (row < seq_q) {
-    const uint8_t* p = mask + (static_cast<size_t>(b) * seq_q + row) * seq_k + col0;
-    const int n = min(64, seq_k - col0);
-    if (n == 64 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+  const int part = threadIdx.x & 7;
+  const int r0 = static_cast<int>(threadIdx.x) >> 3;
+  const int n = min(16, seq_k - (kt * kTile + part * 16));  // columns of this thread that exist (may be <= 0)
+  const int rows = seq_q - qt * kTile - r0;                 // pass i has a row of this thread if 32 i < rows
+  const uint8_t* base = mask + (static_cast<size_t>(b) * seq_q + qt * kTile + r0) * seq_k + kt * kTile + part * 16;
+  uint32_t w[4][4];
+  uint32_t seen = 0u, shown = 0x80808080u;
+  if (n == 16) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    for (int i = 0; i < 4; ++i) {
+      if (32 * i < rows) {
+        row_words16(base + static_cast<size_t>(32 * i) * seq_k, w[i]);
+      } else {
+        w[i][0] = w[i][1] = w[i][2] = w[i][3] = 0u;
+      }
+    }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          // per byte: non-zero?  (b | (b >> 1) | ... folded into bit 0 of each byte)
-          uint32_t x = w[k];
-          x |= x >> 4;
-          x |= x >> 2;
-          x |= x >> 1;
-          x &= 0x01010101u;
-          any |= x != 0u;
-          all &= x == 0x01010101u;
+    for (int i = 0; i < 4; ++i) {
+      if (32 * i < rows) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          seen |= w[i][e];
+          shown &= ((w[i][e] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w[i][e];
         }
       }
-    } else {
-      for (int i = 0; i < n; ++i) {
-        const bool s = p[i] != 0;
-        any |= s;
-        all &= s;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        uint32_t& x = w[i][e >> 2];
+        if ((e & 3) == 0) x = 0u;
+        if (e < n && 32 * i < rows) {
+          const uint32_t byte = base[static_cast<size_t>(32 * i) * seq_k + e];
+          x |= byte << (8 * (e & 3));
+          seen |= byte;
+          if (byte == 0u) shown = 0u;
+        }
       }
     }
   }
-  const int any_cta = __syncthreads_or(any ? 1 : 0);
-  const int all_cta = __syncthreads_and(all ? 1 : 0);
-  if (threadIdx.x == 0)
-    cls[(static_cast<size_t>(b) * gridDim.y + qt) * gridDim.x + kt] = any_cta ? (all_cta ? 1 : 2) : 0;
+  const int any_cta = __syncthreads_or(seen != 0u ? 1 : 0);
+  const int all_cta = __syncthreads_and(shown == 0x80808080u ? 1 : 0);
+  const size_t tile = (static_cast<size_t>(b) * gridDim.y + qt) * gridDim.x + kt;
+  if (threadIdx.x == 0) cls[tile] = any_cta ? (all_cta ? 1 : 2) : 0;
+  if (bits != nullptr && any_cta && !all_cta) {
+    uint32_t* dst = bits + tile * (kTile * kTile / 32);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t v = 0u;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v |= nonzero_bits(w[i][e]) << (4 * e);
+      v |= __shfl_down_sync(0xFFFFFFFFu, v, 1) << 16;
+      if ((part & 1) == 0) dst[(r0 + 32 * i) * 4 + (part >> 1)] = v;
+    }
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, int batch, int seq_q, int seq_k,
+cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, uint32_t* bits, int batch, int seq_q, int seq_k,
                                  cudaStream_t stream) {
   dim3 grid((seq_k + kTile - 1) / kTile, (seq_q + kTile - 1) / kTile, batch);
-  mask_classify_kernel<<<grid, 256, 0, stream>>>(mask, cls, seq_q, seq_k);
+  mask_classify_kernel<<<grid, 256, 0, stream>>>(mask, cls, bits, seq_q, seq_k);
   return cudaGetLastError();
 }
 

@@ -217,6 +217,28 @@ __device__ __forceinline__ int item_id(int k, int n_items) {
   return id < n_items ? id : -1;
 }
 
+// Bits of n (1..128) mask bytes of one row (bit c of w[c / 32]: byte c is non-zero); `vec`: rows are 16-byte aligned.
+// Only calls without room for the tiles' bits in their workspace come here.
+__device__ __forceinline__ void mask_row_bits(const uint8_t* p, int n, bool vec, uint32_t (&w)[4]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t bits = 0u;
+    if (vec && n >= 32 * c + 32) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + 32 * c + 16 * h));
+        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bits |= nonzero_bits(x[e]) << (16 * h + 4 * e);
+      }
+    } else {
+#pragma unroll 1
+      for (int e = 0; e < 32 && 32 * c + e < n; ++e) bits |= (p[32 * c + e] != 0 ? 1u : 0u) << e;
+    }
+    w[c] = bits;
+  }
+}
+
 // What a role needs to walk one item's key tiles.  Causal / unmasked calls: the tiles of slot s are the
 // prefix [0, n[s]).  Dense-mask calls (kMasked): the scheduler warp turns the per-tile classes written by
 // mask_classify_kernel (0 = nothing visible, 1 = all visible, 2 = mixed) into four bit planes over the key
@@ -229,44 +251,58 @@ struct TileList {
   int nvis[2];                    // of which slot s visits
   const volatile uint32_t* planes;  // kMasked only: [n_t / 32][4] bit planes of the flags
   int n0, n1;                     // prefix lengths otherwise
-  // Flags of tile t.  `pw` caches the four plane words of t's group of 32 tiles (the caller scans t upwards
-  // from 0); a group nobody visits is skipped as a whole by advancing t to its last tile.
-  template <bool kMasked>
-  __device__ __forceinline__ uint32_t flag_at(int& t, uint32_t (&pw)[4]) const {
+};
+
+// Walks the tiles of a TileList that at least one slot visits, in ascending order.  Dense masks: by the set bits of
+// the planes, 32 tiles per word, so a tile nobody visits costs nothing.
+template <bool kMasked>
+struct TileCursor {
+  int t = -1;
+  int base = -32;
+  uint32_t todo = 0u, pw[4] = {0u, 0u, 0u, 0u};
+  __device__ __forceinline__ bool next(const TileList& tl) {
     if constexpr (kMasked) {
-      if ((t & 31) == 0) {
-        const volatile uint32_t* g = planes + (t >> 5) * 4;
+      while (todo == 0u) {
+        base += 32;
+        if (base >= tl.n_t) return false;
+        const volatile uint32_t* g = tl.planes + base / 8;
         pw[0] = g[0];
         pw[1] = g[1];
         pw[2] = g[2];
         pw[3] = g[3];
-        if ((pw[0] | pw[2]) == 0u) {
-          t += 31;
-          return 0u;
-        }
+        todo = pw[0] | pw[2];
       }
-      const int sh = t & 31;
-      return ((pw[0] >> sh) & 1u) | (((pw[1] >> sh) & 1u) << 1) | (((pw[2] >> sh) & 1u) << 2) |
-             (((pw[3] >> sh) & 1u) << 3);
+      t = base + __ffs(static_cast<int>(todo)) - 1;
+      todo &= todo - 1u;
+      return true;
     } else {
-      return (t < n0 ? 1u : 0u) | (t < n1 ? 4u : 0u);
+      return ++t < tl.n_t;
     }
   }
-  // Dense masks, one slot's view: bit 0 = slot s visits tile t, bit 1 = it must read mask bytes.  `pv`, `pm`
-  // cache the slot's two plane words of t's group; a group the slot does not visit is skipped as a whole.
-  __device__ __forceinline__ uint32_t slot_flag_at(int s, int& t, uint32_t& pv, uint32_t& pm) const {
-    if ((t & 31) == 0) {
-      const volatile uint32_t* g = planes + (t >> 5) * 4 + 2 * s;
-      pv = g[0];
+  __device__ __forceinline__ bool visits(const TileList& tl, int s) const {
+    if constexpr (kMasked) return ((pw[2 * s] >> (t & 31)) & 1u) != 0u;
+    else return t < (s ? tl.n1 : tl.n0);
+  }
+};
+
+// One slot's view of the same list (dense masks): the tiles slot s visits, and whether mask bytes decide in them.
+struct SlotCursor {
+  int t = -1;
+  int base = -32;
+  uint32_t todo = 0u, pm = 0u;
+  __device__ __forceinline__ bool next(const TileList& tl, int s) {
+    while (todo == 0u) {
+      base += 32;
+      if (base >= tl.n_t) return false;
+      const volatile uint32_t* g = tl.planes + base / 8 + 2 * s;
+      todo = g[0];
       pm = g[1];
-      if (pv == 0u) {
-        t += 31;
-        return 0u;
-      }
     }
-    const int sh = t & 31;
-    return ((pv >> sh) & 1u) | (((pm >> sh) & 1u) << 1);
+    t = base + __ffs(static_cast<int>(todo)) - 1;
+    todo &= todo - 1u;
+    return true;
   }
+  __device__ __forceinline__ bool mixed() const { return ((pm >> (t & 31)) & 1u) != 0u; }
 };
 
 template <int D, bool BF16, bool kMasked>
@@ -516,9 +552,8 @@ prefill_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           ++q_loads[s];
         }
         // K V K V ... of the listed tiles
-        uint32_t pw[4] = {0u, 0u, 0u, 0u};
-        for (int t = 0; t < tl.n_t && ok; ++t) {
-          if (tl.template flag_at<kMasked>(t, pw) == 0u) continue;
+        TileCursor<kMasked> cur;
+        while (ok && cur.next(tl)) {
 #pragma unroll
           for (int h = 0; h < 2 && ok; ++h, ++r) {
             const uint32_t st = r % kStages;
@@ -527,7 +562,7 @@ prefill_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
               break;
             }
             load_tile(h ? &tm_v : &tm_k, kv_addr + st * kTileBytes, &bars[kKvFull + st], a.kv_pos, it.b, it.kvh,
-                      t * kTileN);
+                      cur.t * kTileN);
           }
         }
       }
@@ -599,17 +634,16 @@ prefill_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           }
           if (!ok) break;
           [[maybe_unused]] int s_issued[2] = {0, 0};
-          uint32_t pw[4] = {0u, 0u, 0u, 0u};
-          for (int t = 0, li = 0; t < tl.n_t && ok; ++t) {
-            const uint32_t f = tl.template flag_at<kMasked>(t, pw);
-            if (f == 0u) continue;
+          TileCursor<kMasked> cur;
+          for (int li = 0; ok && cur.next(tl);) {
+            const int t = cur.t;
             const uint32_t rk = r + 2 * li;  // ring position of K of this (the li-th listed) tile
             const uint32_t stk = rk % kStages;
             ++li;
             if (!(ok = mbar_wait(&bars[kKvFull + stk], (rk / kStages) & 1u, abort_flag))) { report_p(a.status, 31); break; }
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-              if (!ok || !(f & (1u << (2 * s)))) continue;
+              if (!ok || !cur.visits(tl, s)) continue;
               // the scores issued last (either slot's) must have been copied out of the S columns
               P_TL(2, t, s * 3 + 0);
               if constexpr (kTwoS) {
@@ -671,17 +705,16 @@ prefill_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             continue;
           }
           [[maybe_unused]] int pv_done[2] = {0, 0};
-          uint32_t pw[4] = {0u, 0u, 0u, 0u};
-          for (int t = 0, li = 0; t < tl.n_t && ok; ++t) {
-            const uint32_t f = tl.template flag_at<kMasked>(t, pw);
-            if (f == 0u) continue;
+          TileCursor<kMasked> cur;
+          for (int li = 0; ok && cur.next(tl);) {
+            const int t = cur.t;
             const uint32_t rv = r + 2 * li + 1;  // ring position of V of this (the li-th listed) tile
             const uint32_t stv = rv % kStages;
             ++li;
             if (!(ok = mbar_wait(&bars[kKvFull + stv], (rv / kStages) & 1u, abort_flag))) { report_p(a.status, 32); break; }
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-              if (!ok || !(f & (1u << (2 * s)))) continue;
+              if (!ok || !cur.visits(tl, s)) continue;
               const bool first_pv = kMasked ? pv_done[s] == 0 : t == 0;
               if (first_pv && items[s] > 0) {
                 // O_s still holds the previous item's result until its epilogue has read it
@@ -763,21 +796,32 @@ prefill_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       }
       const uint8_t* mrow =
           kMasked ? a.mask + (static_cast<size_t>(it.b) * a.seq_q + min(r_glob, a.seq_q - 1)) * a.seq_k : nullptr;
+      // row of the tile bits in key tile 0 (128 rows of 16 bytes per tile)
+      [[maybe_unused]] const uint4* bits_row = nullptr;
+      if constexpr (kMasked) {
+        const int n_qt = (a.seq_q + kTileM - 1) / kTileM, n_kt = (a.seq_k + kTileN - 1) / kTileN;
+        bits_row = reinterpret_cast<const uint4*>(a.bits) +
+                   (static_cast<size_t>(it.b) * n_qt + q0s / kTileM) * n_kt * kTileM + row;
+      }
       float m_ref = -INFINITY;  // reference maximum the stored P and O are relative to
       float l_run = 0.f;
       int jm = 0;  // key tiles this slot has processed in this item (dense masks; else the loop index)
 
-      const int n_iter = kMasked ? tl.n_t : nvis;
-      [[maybe_unused]] uint32_t pv = 0u, pm = 0u;
-      for (int i = 0; i < n_iter; ++i) {
+      [[maybe_unused]] SlotCursor cur;
+      for (int i = 0; kMasked || i < nvis; ++i) {
         bool mixed = false;  // dense masks: the tile needs its mask bytes
         if constexpr (kMasked) {
-          const uint32_t fl = tl.slot_flag_at(s, i, pv, pm);
-          if (!(fl & 1u)) continue;
-          mixed = (fl & 2u) != 0u;
+          if (!cur.next(tl, s)) break;
+          i = cur.t;
+          mixed = cur.mixed();
         }
         const int kv0 = i * kTileN;
         const int j = kMasked ? jm : i;
+        // a mixed tile's bits of this row are requested before the wait for its scores
+        [[maybe_unused]] uint4 mbits = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (kMasked) {
+          if (mixed && a.bits != nullptr) mbits = __ldg(bits_row + static_cast<size_t>(i) * kTileM);
+        }
         P_ACC(acc_c = clock64());
         P_TL(s, j, 0);
         if (!(ok = mbar_wait(&bars[kSFull + s], jt & 1u, abort_flag))) { report_p(a.status, 40); break; }
@@ -800,30 +844,24 @@ prefill_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         // the diagonal and the ragged last tile need it ----
         const bool tail = kv0 + kTileN > a.seq_k;
         const bool diag = !kMasked && a.causal && (kv0 + kTileN - 1 > q0s + off);
-        if (kMasked && mixed) {
-          if (!tail && a.mask_vec) {
-            const uint4* mp = reinterpret_cast<const uint4*>(mrow + kv0);
-#pragma unroll
-            for (int c = 0; c < kTileN / 16; ++c) {
-              const uint4 mv = __ldg(mp + c);
-              const uint32_t w[4] = {mv.x, mv.y, mv.z, mv.w};
-#pragma unroll
-              for (int e = 0; e < 16; ++e)
-                if (((w[e >> 2] >> ((e & 3) * 8)) & 0xFFu) == 0) sr[c * 16 + e] = 0xFF800000u;
-            }
+        if (kMasked ? (mixed || tail) : (tail || diag)) {
+          // the row's visible columns as bits, then one pass over the scores: the byte-reading routes stay small loops
+          // (unrolled over the scores they would put several KB of instructions beside the loop that matters)
+          uint32_t w[4];
+          if (kMasked && mixed) {
+            w[0] = mbits.x; w[1] = mbits.y; w[2] = mbits.z; w[3] = mbits.w;
+            if (a.bits == nullptr) mask_row_bits(mrow + kv0, min(kTileN, a.seq_k - kv0), a.mask_vec != 0, w);
           } else {
+            const int n = min(kTileN - 1, ((!kMasked && a.causal) ? min(a.seq_k - 1, r_glob + off) : a.seq_k - 1) - kv0) + 1;
 #pragma unroll
-            for (int c = 0; c < kTileN; ++c) {
-              const int col = kv0 + c;
-              const bool vis = col < a.seq_k && mrow[col] != 0;
-              if (!vis) sr[c] = 0xFF800000u;
+            for (int c = 0; c < 4; ++c) {
+              const int m = min(32, n - 32 * c);  // visible columns of this word
+              w[c] = m <= 0 ? 0u : 0xFFFFFFFFu >> (32 - m);
             }
           }
-        } else if (tail || diag) {
-          const int lim = (!kMasked && a.causal) ? min(a.seq_k - 1, r_glob + off) : a.seq_k - 1;
 #pragma unroll
           for (int c = 0; c < kTileN; ++c)
-            if (kv0 + c > lim) sr[c] = 0xFF800000u;
+            if (((w[c >> 5] >> (c & 31)) & 1u) == 0u) sr[c] = 0xFF800000u;
         }
 
         // ---- row maximum; move the reference only when it lags by > 2^8 ----

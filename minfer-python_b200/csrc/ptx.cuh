@@ -69,6 +69,13 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   return p;
 }
 
+// One bit per byte of a word (byte 0 -> bit 0): is the byte non-zero?  The sum carries into a byte's top bit when its
+// low seven bits hold anything; the multiply moves the four top bits next to each other.
+__device__ __forceinline__ uint32_t nonzero_bits(uint32_t w) {
+  const uint32_t top = (((w & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) & 0x80808080u;
+  return (top * 0x00204081u) >> 28;
+}
+
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }

@@ -67,12 +67,21 @@ Tensor& scratch(const Tensor& like, void* stream, int64_t purpose, size_t bytes)
   const std::array<int64_t, 3> key = {like.get_device_index(), reinterpret_cast<int64_t>(stream), purpose};
   auto it = g_scratch.find(key);
   if (it == g_scratch.end() || static_cast<size_t>(it->second->numel()) < bytes) {
-    const int64_t n[1] = {static_cast<int64_t>(bytes < (1u << 20) ? (1u << 20) : bytes)};
+    // powers of two, so that the outgrown buffers of a slowly growing series of calls add up to less than the last one
+    int64_t n[1] = {1 << 20};
+    while (static_cast<size_t>(n[0]) < bytes) n[0] *= 2;
     Tensor* t = new Tensor(torch::stable::new_empty(like, {n, 1}, ScalarType::Byte));
     if (it == g_scratch.end()) it = g_scratch.emplace(key, t).first;
     else it->second = t;  // the old buffer stays alive: launches in flight may still use it
   }
   return *it->second;
+}
+
+// Scratch of a dense-mask call: with the tiles' bits (an eighth of the mask's bytes) while that is no more than 256 MB,
+// as for masks up to 2 GB; beyond, the tile classes alone.
+size_t mask_workspace_bytes(int32_t batch, int32_t seq_q, int32_t seq_k) {
+  const size_t with_bits = minfer_attn_prefill_workspace_bytes_bits(batch, seq_q, seq_k);
+  return with_bits <= (size_t{256} << 20) ? with_bits : minfer_attn_prefill_workspace_bytes(batch, seq_q, seq_k);
 }
 
 int dtype_tag(const Tensor& t) {
@@ -138,7 +147,7 @@ void prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor* ma
   p.causal = causal ? 1 : 0;
   p.max_ctas = g_max_ctas;
   void* stream = current_stream();
-  const size_t need = mask != nullptr ? minfer_attn_prefill_workspace_bytes(p.batch, p.seq_q, p.seq_k) : 16;
+  const size_t need = mask != nullptr ? mask_workspace_bytes(p.batch, p.seq_q, p.seq_k) : 16;
   Tensor& ws = scratch(q, stream, /*purpose=*/0, need);
   p.workspace = ws.mutable_data_ptr();
   p.workspace_bytes = static_cast<size_t>(ws.numel());

@@ -21,6 +21,7 @@ ABI_VERSION = 5
 EXPORTS = (
     "minfer_attn_prefill",
     "minfer_attn_prefill_workspace_bytes",
+    "minfer_attn_prefill_workspace_bytes_bits",
     "minfer_attn_decode",
     "minfer_attn_decode_static",
     "minfer_attn_rope_append",
@@ -136,6 +137,8 @@ def _load() -> ctypes.CDLL:
     lib.minfer_attn_prefill.restype = ctypes.c_int
     lib.minfer_attn_prefill_workspace_bytes.argtypes = [ctypes.c_int32] * 3
     lib.minfer_attn_prefill_workspace_bytes.restype = ctypes.c_size_t
+    lib.minfer_attn_prefill_workspace_bytes_bits.argtypes = [ctypes.c_int32] * 3
+    lib.minfer_attn_prefill_workspace_bytes_bits.restype = ctypes.c_size_t
     lib.minfer_attn_decode.argtypes = [ctypes.POINTER(DecodeParams), ctypes.c_void_p]
     lib.minfer_attn_decode.restype = ctypes.c_int
     lib.minfer_attn_decode_static.argtypes = [ctypes.POINTER(DecodeParams), ctypes.c_void_p]

@@ -168,7 +168,11 @@ def _prefill(q, k, v, mask, out, causal: bool, peer_out=()) -> None:
     p.flags = 0
     p.max_ctas = _max_ctas
     # mask tile classes (dense mask) or the persistent kernel's work-item counter (causal)
-    need = _lib.lib.minfer_attn_prefill_workspace_bytes(p.batch, p.seq_q, p.seq_k) if mask is not None else 16
+    need = 16
+    if mask is not None:   # with the mask tiles' bits while they are no more than 256 MB
+        need = _lib.lib.minfer_attn_prefill_workspace_bytes_bits(p.batch, p.seq_q, p.seq_k)
+        if need > 256 << 20:
+            need = _lib.lib.minfer_attn_prefill_workspace_bytes(p.batch, p.seq_q, p.seq_k)
     ws = _workspace_for(q.device, need, _mask_workspace, torch.cuda.current_stream(q.device).cuda_stream)
     p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     with torch.cuda.device(q.device):
@@ -212,7 +216,8 @@ def _workspace_for(device: torch.device, nbytes: int, cache: dict, stream: int =
     idx = (device.index if device.index is not None else torch.cuda.current_device(), stream)
     t = cache.get(idx)
     if t is None or t.numel() < nbytes:
-        t = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        # powers of two: few reallocations over a slowly growing series of calls
+        t = torch.empty(max(1 << (nbytes - 1).bit_length(), 1 << 20), dtype=torch.uint8, device=device)
         cache[idx] = t
     return t
 

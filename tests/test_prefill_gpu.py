@@ -496,3 +496,29 @@ def test_random_shapes_against_the_oracle(kerns, seed):
         check_close_bf16_by_keys(got, want, n_keys, what)    # a sparse random mask makes every row a short one
     else:
         check_close(got, want, what)
+
+
+@pytest.mark.parametrize("L", [1, 15, 127, 130, 143, 257, 272])
+@pytest.mark.parametrize("offset", [0, 5])
+def test_mask_tile_bits_at_unaligned_rows(kerns, L, offset):
+    """Mixed tiles taken from the tiles' bits against the same call that reads mask bytes (no workspace): row lengths
+    and base addresses that put the rows anywhere in a 16-byte chunk, partly filled last tiles, values of true bytes
+    other than 1, empty rows."""
+    from minfer.kernels.torch_ext import _lib
+    B, H, Hkv, D = 2, 4, 2, 64
+    q, k, v = (x.cuda() for x in seeded_qkv(7 + L, B, H, Hkv, L, L, D, torch.float16))
+    g = torch.Generator().manual_seed(L + offset)
+    m = (torch.rand(B, 1, L, L, generator=g) < 0.4).to(torch.uint8) * torch.randint(1, 256, (B, 1, L, L), generator=g, dtype=torch.uint8)
+    m[:, :, L // 2] = 0
+    buf = torch.zeros(offset + m.numel(), dtype=torch.uint8, device="cuda")
+    buf[offset:] = m.flatten().cuda()
+    mask = buf[offset:]
+    outs = []
+    for need in (_lib.lib.minfer_attn_prefill_workspace_bytes_bits(B, L, L), 0):
+        ws = torch.full((need,), 0xFF, dtype=torch.uint8, device="cuda") if need else None
+        out = torch.full((B, H, L, D), float("nan"), dtype=torch.float16, device="cuda")
+        assert _c_abi_call(q, k, v, out, mask=mask, causal=False, ws=ws) == 0
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    check_close(outs[0], O.attention_f64(q.cpu(), k.cpu(), v.cpu(), mask=m != 0), f"bits L={L} offset={offset}")
