@@ -159,12 +159,13 @@ size_t minfer_attn_prefill_workspace_bytes_bits(int32_t batch, int32_t seq_q, in
  * attends keys [0, lens[b]); entries beyond lens[b] are never read.  A
  * sequence with lens[b] == 0 yields zeros.
  *
- * The KV range of a sequence is cut into chunks of `chunk` keys, each handled
- * by its own thread block (split-KV); partial results go through `workspace`,
- * a device buffer of at least minfer_attn_decode_workspace_bytes() bytes that
- * the caller owns (any content); a second, small kernel merges the splits of
- * every sequence and writes `out`.  chunk == 0 lets the library choose; otherwise it must be a
- * positive multiple of 64.
+ * The KV range of a sequence is shared by several thread blocks (split-KV).
+ * chunk == 0 lets the library choose how: usually a cluster of blocks that merge
+ * through each other's shared memory.  chunk > 0, a multiple of 64: one block per
+ * `chunk` keys, partial results through `workspace`, and a second, small kernel that merges
+ * the chunks of every sequence and writes `out`.  Either way `workspace` is a device
+ * buffer of at least minfer_attn_decode_workspace_bytes() bytes that the caller
+ * owns (any content).
  *
  * kv_format == MINFER_ATTN_KV_Q8_0: the caches hold GGML Q8_0 blocks (the
  * reference's block_q8_0, csrc/common/types.hpp:141-146): a cache row is
@@ -221,7 +222,8 @@ size_t minfer_attn_decode_workspace_bytes(int32_t batch, int32_t n_heads,
                                           int32_t max_len, int32_t head_dim,
                                           int32_t chunk);
 
-/* The chunk minfer_attn_decode() uses when params->chunk == 0. */
+/* The chunk that minfer_attn_decode() sizes its workspace by (and uses where it cuts a sequence into chunks) when
+ * params->chunk == 0. */
 int32_t minfer_attn_decode_default_chunk(int32_t batch, int32_t n_kv_heads,
                                          int32_t max_len);
 

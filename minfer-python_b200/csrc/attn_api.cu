@@ -145,6 +145,28 @@ int32_t default_chunk(int32_t batch, int32_t n_kv_heads, int32_t max_len) {
   return c;
 }
 
+// 160 MB of keys and values at full length
+bool decode_is_large(int64_t pairs, int64_t max_len, int64_t row_bytes) { return pairs * max_len * row_bytes * 2 > (int64_t{160} << 20); }
+
+// Blocks (one cluster) per (sequence, kv head) of a decode call, or 0: chunks, and a second kernel that merges them.
+// The lengths are on the device, so the rule knows the padded length only.
+//   A block costs about 4 us beside its keys (launch, the chain length -> keys -> scores, merge), and two fit an SM.
+//   While the caches hold little, a call is one such latency: as many blocks as one wave takes (296), no more.  Measured
+//   (us, 1 / 2 / 4 / 8 / 16 blocks): 1 sequence, 8 kv heads, 777 keys, D=128 7.5 / 6.5 / 5.4 / 4.7 / 4.7; 8 sequences of
+//   513-640, D=64 6.8 / 6.9 / 6.4 / 6.3 / 13.6; 8 of 2000-4096, D=128 32 / 23 / 19.7 / 21.2 / 33; 32 of 300 9.3 / 14.2 / 21 / ...
+//   Large caches (worth 25 us of bandwidth and more) are taken in several waves, so that a batch of ragged lengths
+//   leaves no long tail (with the longest sequences first, see sequence_by_length): 64 sequences of 512-8192, 8 kv heads
+//   164 / 165 / 176 / 206; 24 of 100-6000 72 / 54.3 / 54.2 / 63; Q8_0, 64 of 512-8192 153 / 107 / 121 / 153.
+//   A handful of heads over a very long cache would leave most SMs without a block: chunks then.
+int decode_parts(int64_t batch, int64_t n_kv_heads, int64_t max_len, int64_t row_bytes) {
+  const int64_t pairs = batch * n_kv_heads;
+  if (pairs <= 4 && max_len >= 32768) return 0;
+  const int64_t limit = decode_is_large(pairs, max_len, row_bytes) ? 1024 : 2 * 148;
+  int parts = 1;
+  while (parts < 16 && pairs * parts * 2 <= limit && max_len >= 64 * parts * 2) parts *= 2;
+  return parts;
+}
+
 }  // namespace
 
 int cuda_result(cudaError_t e) {
@@ -422,8 +444,18 @@ int minfer_attn_decode(const MinferAttnDecodeParams* p, void* stream) {
   a.group = group;
   a.chunk = chunk;
   a.n_split = (p->max_len + chunk - 1) / chunk;
-  a.part_o = static_cast<float*>(p->workspace);
-  a.part_ml = a.part_o + static_cast<size_t>(p->batch) * p->n_heads * a.n_split * p->head_dim;
+  const int64_t pairs = static_cast<int64_t>(p->batch) * p->n_kv_heads;
+  const int64_t row_bytes = 2 * p->head_dim;  // of a 16-bit cache for Q8_0 too: both split a sequence alike, so their sums agree bit for bit
+  // (an explicit chunk keeps its meaning: one block per chunk, partial results through the workspace)
+  const int parts = p->chunk == 0 ? decode_parts(p->batch, p->n_kv_heads, p->max_len, row_bytes) : 0;
+  if (parts > 0) {
+    a.n_split = parts;
+    // ranking the batch costs a block about 1 us: where the call is one wave there is no order to choose
+    a.by_length = (p->batch > 1 && p->batch <= 256 && pairs * parts > 2 * 148 && decode_is_large(pairs, p->max_len, row_bytes)) ? 1 : 0;
+  } else {
+    a.part_o = static_cast<float*>(p->workspace);
+    a.part_ml = a.part_o + static_cast<size_t>(p->batch) * p->n_heads * a.n_split * p->head_dim;
+  }
   for (int i = 0; i < 2; ++i) {
     a.q_stride[i] = p->q_stride[i];
     a.out_stride[i] = p->out_stride[i];

@@ -17,6 +17,25 @@ constexpr int32_t kStatusBadPosition = 102;  // a cache row outside [0, max_len)
 // and maps it to MINFER_ATTN_OK / MINFER_ATTN_ECUDA.
 int cuda_result(cudaError_t e);
 
+// Launch configuration with programmatic stream serialisation (see grid_dependency_wait in ptx.cuh), optionally clusters.
+struct LaunchAttrs {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  explicit LaunchAttrs(cudaStream_t stream) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  LaunchAttrs(const LaunchAttrs&) = delete;
+  void cluster(int x) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim = {static_cast<unsigned>(x), 1u, 1u};
+    cfg.numAttrs = 2;
+  }
+};
+
 // Kernel-side view of a prefill call (tensor maps travel separately).
 struct PrefillArgs {
   void* out;
@@ -89,7 +108,8 @@ struct DecodeArgs {
   const void* v;
   const int32_t* lens;
   void* out;
-  float* part_o;   // [batch, n_heads, n_split, head_dim] fp32, unnormalised
+  float* part_o;   // [batch, n_heads, n_split, head_dim] fp32, unnormalised; null: the blocks of a sequence form a
+                   // cluster of n_split, share its keys evenly and merge through each other's shared memory
   float* part_ml;  // [batch, n_heads, n_split, 2] running max (log2 domain) and sum
   int64_t q_stride[2];
   int64_t kv_stride[3];   // elements; for a Q8_0 cache: bytes (batch, head), rows contiguous
@@ -97,7 +117,8 @@ struct DecodeArgs {
   int32_t batch, n_heads, n_kv_heads, max_len;
   int32_t group;
   int32_t chunk;    // keys per thread block
-  int32_t n_split;  // ceil(max_len / chunk)
+  int32_t n_split;  // ceil(max_len / chunk), or the cluster size
+  int32_t by_length;  // blocks take the sequences in order of descending length (batch <= 256)
   float scale_log2;
   const int32_t* block_table;  // paged cache: [batch, table_stride] page indices; kv_stride[0] is then per page
   int32_t page_size, table_stride;

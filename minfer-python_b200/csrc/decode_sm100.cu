@@ -5,36 +5,41 @@
 // layout [batch, n_kv_heads, max_len, head_dim] is the one its model skeleton
 // allocates (src/minfer/core.py:105-127).
 //
-// Kernel 1 (decode_split_kernel): grid (n_split, n_kv_heads, batch).  A thread
-// block streams `chunk` keys of one (sequence, kv head) and serves all `group`
-// query heads of that kv head at once, so every cache byte is read once.  Each
-// warp runs a private cp.async ring of 16-key tiles (128-bit loads, rows of the
-// cache are contiguous, so a warp instruction covers whole 256/128-byte rows)
-// and keeps its own online-softmax state; the grouped query heads occupy the
-// 16 rows of m16n8k16 tensor-core tiles so the arithmetic stays far below the
-// memory time.  The warps' states are merged through shared memory and written
-// as one fp32 partial (max, sum, unnormalised output) per (query head, split).
+// decode_kernel: grid (parts, n_kv_heads, batch).  A thread block streams a part of the keys of one (sequence, kv
+// head) and serves all `group` query heads at once, so every cache byte is read once.  Each warp runs a private
+// cp.async ring of 16-key tiles (128-bit loads, rows of the cache are contiguous, so a warp instruction covers
+// whole 256/128-byte rows) and keeps its own online-softmax state.
+//
+// The products are taken transposed: S^T = K Q^T and O^T = V^T P^T, keys (dimensions) as the 16 rows of an
+// m16n8k16 tile and query heads as its 8 columns, because a GQA group is rarely more than 8.  With the heads as rows
+// half of every MMA, of the accumulators and of the exponentials belonged to rows that do not exist; transposed, a
+// 16-key tile takes half the MMAs and 4 exponentials per lane (groups of 9-16 take two column tiles).  P^T comes
+// from S^T by two 8x8 transposes (movmatrix) per tile.  The reference maximum moves only when a score exceeds it by
+// 2^8, so ordinary tiles need no reduction over lanes.  (Counted from the source, a Q8_0 tile takes some 430 warp
+// instructions, 780 were measured before;
+// the batch-64 Q8_0 call 147 -> 107 us, 5.2 of 6.5 TB/s.)
+//
+// The blocks of one (sequence, kv head) form a cluster: they share the sequence's actual tiles evenly - a padded
+// cache has no empty blocks - and each pushes its partial output into the shared memory of the block that finishes
+// that slice of the result, so one launch does the whole call and no partial result touches memory (split-KV with a
+// second, merging kernel took 4.2 + 2.8 us where this takes 4.7 together, and 6 us behind the batch-64 call).  Calls
+// with an explicit chunk, or a handful of heads over a very long cache (see decode_parts in attn_api.cu), write partials to the workspace
+// instead, merged by decode_combine_kernel.
 //
 // Q8 = true: the caches hold GGML Q8_0 blocks (32 int8 + one fp16 scale, 34 bytes;
 // the reference's block_q8_0, src/minfer/kernels/torch_ext/csrc/common/types.hpp:141-146).
 // The raw bytes of a 16-key tile are contiguous in the cache and ride the same
-// cp.async ring; every lane then builds its tensor-core B fragments straight from
+// cp.async ring; every lane then builds its tensor-core fragments straight from
 // the raw rows in shared memory - two int8 dropped into the mantissas of a pair of
 // halves, the bias subtracted, one multiply by the block's scale - so each value
 // is (16-bit type)(q * d), rounded once, exactly as the reference's
 // dequant_row_q8_0<half> produces it (csrc/quants/impl.cpp:1153-1166), and no
-// 16-bit copy of the tile is ever written.  K keeps the key and dimension order of
-// the 16-bit path, so the scores are the same bits; for V a lane takes four
-// consecutive dimensions of each block (the output columns come out permuted
-// inside a block and are put back in the merge), which leaves every sum over the
-// keys as it was.  Cache bytes per key drop from 4 D to 2.125 D.
+// 16-bit copy of the tile is ever written.  A lane takes four consecutive
+// dimensions at a time: for K that permutes the 16 summands of an MMA (whose sum
+// does not depend on their order), for V the rows of the output inside a block (put
+// back in the merge), so every result has the bits of the 16-bit path.  Cache bytes per key drop from 4 D to 2.125 D.
 //
-// Kernel 2 (decode_combine_kernel): grid (n_heads, batch) merges the partials
-// of the ceil(len / chunk) splits of a sequence and writes the 16-bit output.
-// (A one-launch form - every thread block takes a ticket from a counter after
-// writing its partial and the last one of a (sequence, kv head) merges - was
-// built and measured: the fence and the atomic add about 2 us to every 12 us
-// thread block, which costs more than this second launch does.)
+// decode_combine_kernel: grid (n_heads, batch) merges the partials of the ceil(len / chunk) chunks of a sequence.
 #include "attn_internal.h"
 #include "ptx.cuh"
 
@@ -48,6 +53,8 @@ namespace {
 
 constexpr int kWarps = 4;
 constexpr int kStages = 3;
+constexpr int kMaxParts = 16;    // blocks per cluster (above 8: the non-portable size, which sm_100 has)
+constexpr int kMaxRanked = 256;  // sequences a block ranks by length
 // Q8_0: thread blocks per SM and ring depth (raw tiles are about half the bytes of 16-bit ones)
 #ifndef MINFER_ATTN_Q8_CTAS
 #define MINFER_ATTN_Q8_CTAS 3
@@ -56,6 +63,21 @@ constexpr int kStages = 3;
 #define MINFER_ATTN_Q8_STAGES 4
 #endif
 constexpr int kTileKeys = 16;
+constexpr float kMoveThreshold = 8.0f;  // log2 units
+
+// Shared memory of a decode block: the warps' rings (reused for their partial outputs), then what the merges need.
+template <int D, bool Q8, int NT>
+struct Layout {
+  static constexpr int kStages = Q8 ? MINFER_ATTN_Q8_STAGES : minfer_attn::kStages;
+  static constexpr int kTileBytes = Q8 ? kTileKeys * (D / 32) * 34 : kTileKeys * D * 2;
+  static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
+  static constexpr int kRingBytes = kWarps * kWarpBytes;
+  static constexpr int kWmlBytes = kWarps * 8 * NT * 8;
+  static constexpr int kPartBytes = 8 * NT * D * 4;
+  static constexpr int kBytes = kRingBytes + kWmlBytes + kPartBytes + kMaxParts * 8 * NT * 8;
+  static_assert(kWarpBytes >= 8 * NT * (D + 4) * 4, "the per-warp ring also holds the warp's partial output");
+  static_assert(kRingBytes >= (kMaxRanked + 2) * 4, "the ranking by length borrows the ring");
+};
 
 // kept out of line: the error path must not cost the streaming loop registers
 __device__ __noinline__ void report_bad_page(int32_t* status, int b, int slot, int page) {
@@ -93,6 +115,47 @@ __device__ __forceinline__ Q8Scale<BF16> q8_scale(uint32_t d_lo, uint32_t d_hi) 
   }
   return r;
 }
+template <bool BF16>
+__device__ __forceinline__ Q8Scale<BF16> q8_scale_pair(uint32_t d) {  // both bit patterns in one word
+  if constexpr (BF16) return q8_scale<true>(d & 0xFFFFu, d >> 16);
+  Q8Scale<BF16> r;
+  if constexpr (!BF16) r.h2 = d;
+  return r;
+}
+// four bytes of a Q8_0 row in shared memory: a block's values start 2 bytes behind a multiple of 4 in every other block
+__device__ __forceinline__ uint32_t ld_q8_word(const uint8_t* p, bool aligned4) {
+  if (aligned4) return *reinterpret_cast<const uint32_t*>(p);
+  return static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(p)) |
+         (static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(p + 2)) << 16);
+}
+
+// The sequence that is i-th when the batch is ordered by descending length (ties by index); every block finds its own.
+// Blocks start in grid order, so the long sequences start first and the last wave holds the short ones.  Four lengths
+// per shared-memory read, the reads of one sequence dealt out over the lanes a small batch leaves free.  Returns the
+// sequence and its length.
+__device__ __forceinline__ int2 sequence_by_length(const int32_t* lens, int batch, int i, int* scratch, int tid) {
+  const int n4 = (batch + 3) / 4;
+  for (int t = tid; t < 4 * n4; t += kWarps * 32) scratch[t] = t < batch ? lens[t] : -1;
+  int lanes = 1;  // per sequence
+  while (lanes < 16 && 2 * lanes * batch <= kWarps * 32) lanes *= 2;
+  __syncthreads();
+  for (int t0 = 0; t0 < batch; t0 += kWarps * 32 / lanes) {
+    const int t = t0 + tid / lanes;
+    const int mine = t < batch ? scratch[t] : 0;
+    int rank = 0;
+    for (int u = tid % lanes; u < n4; u += lanes) {
+      const int4 x = reinterpret_cast<const int4*>(scratch)[u];
+      // lengths before `t` count when equal, those behind it do not
+      rank += (x.x >= mine + (4 * u >= t ? 1 : 0)) + (x.y >= mine + (4 * u + 1 >= t ? 1 : 0)) +
+              (x.z >= mine + (4 * u + 2 >= t ? 1 : 0)) + (x.w >= mine + (4 * u + 3 >= t ? 1 : 0));
+    }
+    for (int d = lanes >> 1; d > 0; d >>= 1) rank += __shfl_xor_sync(0xFFFFFFFFu, rank, d);
+    if (t < batch && rank == i && tid % lanes == 0) *reinterpret_cast<int2*>(&scratch[kMaxRanked]) = make_int2(t, mine);
+  }
+  __syncthreads();
+  return *reinterpret_cast<const int2*>(&scratch[kMaxRanked]);
+}
+
 template <bool BF16, int I0, int I1>
 __device__ __forceinline__ uint32_t q8_pair(uint32_t src, const Q8Scale<BF16>& d) {
   if constexpr (BF16) {
@@ -111,36 +174,56 @@ __device__ __forceinline__ uint32_t q8_pair(uint32_t src, const Q8Scale<BF16>& d
 }
 
 // Paged: the caches are pools of pages reached through a.block_table (a separate instantiation, so that the
-// contiguous form keeps its registers).
-template <int D, bool BF16, bool Q8, bool Paged>
-__global__ void __launch_bounds__(kWarps * 32, Q8 ? MINFER_ATTN_Q8_CTAS : 2) decode_split_kernel(const DecodeArgs a) {
-  constexpr int kSt = Q8 ? MINFER_ATTN_Q8_STAGES : kStages;
-  constexpr int kRowBytes = D * 2;
-  constexpr int kTileBytes = kTileKeys * kRowBytes;        // one of K or V, 16-bit
+// contiguous form keeps its registers).  NT: 8-column tiles the query heads of a kv head fill (1: group <= 8).
+template <int D, bool BF16, bool Q8, bool Paged, int NT>
+__global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_CTAS : 2) decode_kernel(const DecodeArgs a) {
+  using L = Layout<D, Q8, NT>;
+  constexpr int kSt = L::kStages;
+  constexpr int kTileBytes = L::kTileBytes;                // one of K or V
   constexpr int kChunksPerRow = D / 8;                     // 16-byte chunks
   constexpr int kLoadsPerLane = kTileKeys * kChunksPerRow / 32;
   // Q8_0: raw rows of D/32 blocks of 34 bytes; a 16-row tile is one contiguous, 16-byte aligned span
   constexpr int kQRowBytes = (D / 32) * 34;
-  constexpr int kQTileBytes = kTileKeys * kQRowBytes;      // 2176 (D=128) / 1088 (D=64): multiples of 16
-  constexpr int kQChunks = kQTileBytes / 16;
+  constexpr int kQChunks = kTileKeys * kQRowBytes / 16;
   constexpr int kQLoadsPerLane = (kQChunks + 31) / 32;
-  // per warp: the ring of raw tiles
-  constexpr int kWarpBytes = kSt * 2 * (Q8 ? kQTileBytes : kTileBytes);
+  constexpr int kWarpBytes = L::kWarpBytes;
 
   extern __shared__ __align__(128) uint8_t smem[];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const int split = blockIdx.x;
   const int kvh = blockIdx.y;
-  const int b = blockIdx.z;
+  const bool clustered = a.part_o == nullptr;
+  const int part = blockIdx.x;       // which piece of the sequence
+  const int n_parts = gridDim.x;
 
-  const int len = min(a.lens[b], a.max_len);
-  const int c0 = split * a.chunk;
-  if (c0 >= len) return;
-  const int c1 = min(len, c0 + a.chunk);
-  const int nt = (c1 - c0 + kTileKeys - 1) / kTileKeys;
+  grid_launch_dependents();
+  if (clustered && n_parts > 1) cluster_arrive();  // awaited before the first access to another block's shared memory
+  grid_dependency_wait();
+
+  // ---- which sequence: in order, or the i-th longest (a.by_length: few enough sequences to rank them here) ----
+  int b = blockIdx.z, len;
+  if (a.by_length) {
+    const int2 x = sequence_by_length(a.lens, a.batch, b, reinterpret_cast<int*>(smem), tid);
+    b = x.x;
+    len = x.y;
+  } else {
+    len = a.lens[b];
+  }
+  len = max(0, min(len, a.max_len));
+  // ---- the keys of this block: an even share of the sequence's tiles, or the part-th chunk ----
+  int c0, c1;
+  if (clustered) {
+    const int nt_seq = (len + kTileKeys - 1) / kTileKeys;
+    c0 = static_cast<int>(static_cast<unsigned>(nt_seq) * static_cast<unsigned>(part) / static_cast<unsigned>(n_parts)) * kTileKeys;
+    c1 = min(len, static_cast<int>(static_cast<unsigned>(nt_seq) * static_cast<unsigned>(part + 1) / static_cast<unsigned>(n_parts)) * kTileKeys);
+  } else {
+    c0 = part * a.chunk;
+    if (c0 >= len) return;
+    c1 = min(len, c0 + a.chunk);
+  }
+  const int nt = c1 > c0 ? (c1 - c0 + kTileKeys - 1) / kTileKeys : 0;
   const int nt_w = (nt > warp) ? (nt - warp + kWarps - 1) / kWarps : 0;
 
   uint8_t* wsm = smem + warp * kWarpBytes;
@@ -150,7 +233,7 @@ __global__ void __launch_bounds__(kWarps * 32, Q8 ? MINFER_ATTN_Q8_CTAS : 2) dec
   // (Everything is recomputed per tile from kernel parameters, which costs no registers between tiles.)
   auto tile_offset = [&](int key0) -> size_t {
     constexpr size_t kUnit = Q8 ? 1 : 2;  // Q8_0 strides are in bytes
-    const size_t row_bytes = Q8 ? static_cast<size_t>((D / 32) * 34) : 2 * static_cast<size_t>(a.kv_stride[2]);
+    const size_t row_bytes = Q8 ? static_cast<size_t>(kQRowBytes) : 2 * static_cast<size_t>(a.kv_stride[2]);
     const size_t head_off = kUnit * static_cast<size_t>(kvh) * a.kv_stride[1];
     if constexpr (Paged) {
       const int slot = key0 / a.page_size;
@@ -170,12 +253,12 @@ __global__ void __launch_bounds__(kWarps * 32, Q8 ? MINFER_ATTN_Q8_CTAS : 2) dec
     if (i < nt_w) {
       const int key0 = c0 + (warp + i * kWarps) * kTileKeys;
       const size_t toff = tile_offset(key0);
+      uint8_t* dst_k = wsm + (i % kSt) * 2 * kTileBytes;
+      uint8_t* dst_v = dst_k + kTileBytes;
       if constexpr (Q8) {
         // strides of a Q8_0 cache are in bytes; rows are contiguous
         const uint8_t* kq = reinterpret_cast<const uint8_t*>(a.k) + toff;
         const uint8_t* vq = reinterpret_cast<const uint8_t*>(a.v) + toff;
-        uint8_t* dst_k = wsm + (i % kSt) * 2 * kQTileBytes;
-        uint8_t* dst_v = dst_k + kQTileBytes;
         // bytes of live rows in this tile (rows beyond the sequence are neither read nor used)
         const int live = min(kTileKeys, c1 - key0) * kQRowBytes;
 #pragma unroll
@@ -187,55 +270,67 @@ __global__ void __launch_bounds__(kWarps * 32, Q8 ? MINFER_ATTN_Q8_CTAS : 2) dec
             cp_async_16(dst_v + ch * 16, vq + (pred ? ch * 16 : 0), pred);
           }
         }
-        cp_async_commit();
-        return;
-      }
-      uint8_t* dst_k = wsm + (i % kSt) * 2 * kTileBytes;
-      uint8_t* dst_v = dst_k + kTileBytes;
+      } else {
 #pragma unroll
-      for (int t = 0; t < kLoadsPerLane; ++t) {
-        const int idx = t * 32 + lane;
-        const int row = idx / kChunksPerRow;
-        const int chunk = idx % kChunksPerRow;
-        const bool pred = key0 + row < c1;
-        const size_t goff = toff + static_cast<size_t>(pred ? row : 0) * row_stride_bytes + chunk * 16;
-        cp_async_16(dst_k + swz<D>(row, chunk), reinterpret_cast<const uint8_t*>(a.k) + goff, pred);
-        cp_async_16(dst_v + swz<D>(row, chunk), reinterpret_cast<const uint8_t*>(a.v) + goff, pred);
+        for (int t = 0; t < kLoadsPerLane; ++t) {
+          const int idx = t * 32 + lane;
+          const int row = idx / kChunksPerRow;
+          const int chunk = idx % kChunksPerRow;
+          const bool pred = key0 + row < c1;
+          const size_t goff = toff + static_cast<size_t>(pred ? row : 0) * row_stride_bytes + chunk * 16;
+          cp_async_16(dst_k + swz<D>(row, chunk), reinterpret_cast<const uint8_t*>(a.k) + goff, pred);
+          cp_async_16(dst_v + swz<D>(row, chunk), reinterpret_cast<const uint8_t*>(a.v) + goff, pred);
+        }
       }
     }
     cp_async_commit();
   };
 
+  if (a.by_length) __syncthreads();  // the ranking's scratch is the ring's memory
 #pragma unroll
   for (int s = 0; s < kSt - 1; ++s) issue_tile(s);
 
-  // ---- Q fragments: rows = query heads of this kv head (zero beyond group) ----
+  // ---- Q^T fragments (B operand): columns = query heads of this kv head (zero beyond group).  Q8_0: the 16 k slots
+  // of a step hold its dimensions in another order (slots 2t, 2t+1, 2t+8, 2t+9 of lane t: dimensions 4t .. 4t+3), so that a lane's
+  // four K values are four consecutive bytes; an MMA's sum over its 16 slots does not depend on their order. ----
   const int g0 = lane >> 2;
   const int tq = lane & 3;
-  uint32_t qf[D / 16][4];
+  uint32_t qf[NT][D / 16][2];
   {
     const uint8_t* qb = reinterpret_cast<const uint8_t*>(a.q) + 2 * static_cast<size_t>(b) * a.q_stride[0];
-    const int h0 = kvh * a.group + g0;
-    const int h1 = h0 + 8;
-    const uint8_t* q0p = qb + 2 * static_cast<size_t>(h0) * a.q_stride[1];
-    const uint8_t* q1p = qb + 2 * static_cast<size_t>(h1) * a.q_stride[1];
-    const bool v0 = g0 < a.group;
-    const bool v1 = g0 + 8 < a.group;
 #pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-      const int d = ks * 16 + tq * 2;
-      qf[ks][0] = v0 ? *reinterpret_cast<const uint32_t*>(q0p + 2 * d) : 0u;
-      qf[ks][1] = v1 ? *reinterpret_cast<const uint32_t*>(q1p + 2 * d) : 0u;
-      qf[ks][2] = v0 ? *reinterpret_cast<const uint32_t*>(q0p + 2 * (d + 8)) : 0u;
-      qf[ks][3] = v1 ? *reinterpret_cast<const uint32_t*>(q1p + 2 * (d + 8)) : 0u;
+    for (int n = 0; n < NT; ++n) {
+      const int g = g0 + 8 * n;
+      const bool live = g < a.group;
+      const uint8_t* qp = qb + 2 * static_cast<size_t>(kvh * a.group + (live ? g : 0)) * a.q_stride[1];
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks) {
+        if constexpr (Q8) {
+          const uint2 x = *reinterpret_cast<const uint2*>(qp + 2 * (ks * 16 + tq * 4));
+          qf[n][ks][0] = live ? x.x : 0u;
+          qf[n][ks][1] = live ? x.y : 0u;
+        } else {
+          const uint32_t x = *reinterpret_cast<const uint32_t*>(qp + 2 * (ks * 16 + tq * 2));
+          const uint32_t y = *reinterpret_cast<const uint32_t*>(qp + 2 * (ks * 16 + tq * 2 + 8));
+          qf[n][ks][0] = live ? x : 0u;
+          qf[n][ks][1] = live ? y : 0u;
+        }
+      }
     }
   }
 
-  float oacc[D / 8][4];
+  // O^T: oacc[n][m][0..3] = (row g0, heads 2 tq, 2 tq + 1), (row g0 + 8, the same) of the m-th 16-row tile
+  float oacc[NT][D / 16][4];
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n) oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY};  // log2 domain (already scaled)
-  float l_run[2] = {0.f, 0.f};              // this thread's share of the row sums
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int m = 0; m < D / 16; ++m) oacc[n][m][0] = oacc[n][m][1] = oacc[n][m][2] = oacc[n][m][3] = 0.f;
+  float m_ref[NT][2], l_run[NT][2];  // per head: reference maximum (log2 domain), this lane's share of the row sum
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    m_ref[n][0] = m_ref[n][1] = -INFINITY;
+    l_run[n][0] = l_run[n][1] = 0.f;
+  }
   const float sl2 = a.scale_log2;
 
   // ldmatrix lane roles
@@ -248,199 +343,267 @@ __global__ void __launch_bounds__(kWarps * 32, Q8 ? MINFER_ATTN_Q8_CTAS : 2) dec
     issue_tile(i + kSt - 1);
 
     const int key0 = c0 + (warp + i * kWarps) * kTileKeys;
-    // ---- S[16 heads x 16 keys] = Q K^T ----
-    float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    [[maybe_unused]] const uint8_t* raw_k = wsm + (i % kSt) * 2 * kQTileBytes;  // Q8: this tile's raw K rows, then V
-    [[maybe_unused]] uint32_t sv = 0;
+    // ---- S^T[16 keys x 8 heads] = K Q^T ----
+    // (two accumulators: half the length of the chain of dependent MMAs)
+    float s[NT][4], s2[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[n][e] = s2[n][e] = 0.f;
+    [[maybe_unused]] const uint8_t* raw_k = wsm + (i % kSt) * 2 * kTileBytes;  // Q8: this tile's raw K rows, then V
+    [[maybe_unused]] const uint32_t sk = wsm_u32 + (i % kSt) * 2 * kTileBytes;
     if constexpr (Q8) {
-      // B fragments from the raw rows: lane (g0, tq) holds keys g0 / g0 + 8 and, per 16-dimension step, the pairs
-      // at 2 tq and 2 tq + 8 - two-byte loads (the blocks' 34 bytes leave nothing better aligned), the four lanes
-      // of a key reading 8 consecutive bytes.  Rows beyond the chunk were zero-filled by the copy (scale 0).
+      // A fragments from the raw rows: keys g0 / g0 + 8, per 16-dimension step four consecutive bytes.  Rows beyond
+      // the chunk were zero-filled by the copy (their scores are masked below).
 #pragma unroll
       for (int blk = 0; blk < D / 32; ++blk) {
+        uint32_t kf[2][4];
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-          const uint8_t* bp = raw_k + (g0 + 8 * nb) * kQRowBytes + blk * 34;
+        for (int kk = 0; kk < 2; ++kk) {
+          const uint8_t* bp = raw_k + (g0 + 8 * kk) * kQRowBytes + blk * 34;
           const uint32_t db = *reinterpret_cast<const uint16_t*>(bp);
           const Q8Scale<BF16> d = q8_scale<BF16>(db, db);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint32_t u0 = *reinterpret_cast<const uint16_t*>(bp + 2 + 16 * h + 2 * tq);
-            const uint32_t u1 = *reinterpret_cast<const uint16_t*>(bp + 2 + 16 * h + 8 + 2 * tq);
-            mma_16816<BF16>(sacc[nb], qf[2 * blk + h], q8_pair<BF16, 0, 1>(u0 ^ 0x8080u, d),
-                            q8_pair<BF16, 0, 1>(u1 ^ 0x8080u, d));
+            const uint32_t x = ld_q8_word(bp + 2 + 16 * h + 4 * tq, (blk & 1) != 0) ^ 0x80808080u;
+            kf[h][kk] = q8_pair<BF16, 0, 1>(x, d);
+            kf[h][2 + kk] = q8_pair<BF16, 2, 3>(x, d);
           }
         }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int n = 0; n < NT; ++n) mma_16816<BF16>(h ? s2[n] : s[n], kf[h], qf[n][2 * blk + h][0], qf[n][2 * blk + h][1]);
       }
     } else {
-      const uint32_t sk = wsm_u32 + (i % kSt) * 2 * kTileBytes;
-      sv = sk + kTileBytes;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t r0, r1, r2, r3;
-        const int key = (lm_mi >> 1) * 8 + lm_r;
-        const int chunk = 2 * ks + (lm_mi & 1);
-        ldmatrix_x4(sk + swz<D>(key, chunk), r0, r1, r2, r3);
-        mma_16816<BF16>(sacc[0], qf[ks], r0, r1);
-        mma_16816<BF16>(sacc[1], qf[ks], r2, r3);
+        uint32_t kf[4];
+        ldmatrix_x4(sk + swz<D>((lm_mi & 1) * 8 + lm_r, 2 * ks + (lm_mi >> 1)), kf[0], kf[1], kf[2], kf[3]);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma_16816<BF16>((ks & 1) ? s2[n] : s[n], kf, qf[n][ks][0], qf[n][ks][1]);
       }
     }
 
-    // ---- scale, mask the ragged end, online softmax ----
-    const bool partial = key0 + kTileKeys > c1;
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[n][e] += s2[n][e];
+
+    // ---- online softmax over the keys: x = s * scale - reference; the reference moves only when a score exceeds it
+    // by 2^8 (weights stay below 256, sums in fp32), so that ordinary tiles need no reduction over the lanes ----
+    const bool partial = key0 + kTileKeys > c1;
+    const bool dead0 = partial && key0 + g0 >= c1, dead1 = partial && key0 + g0 + 8 >= c1;
+    float x[NT][4];
+    bool move = false;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        float s = sacc[nb][e] * sl2;
-        if (partial && (key0 + nb * 8 + tq * 2 + (e & 1) >= c1)) s = -INFINITY;
-        sacc[nb][e] = s;
+        x[n][e] = fmaf(s[n][e], sl2, -m_ref[n][e & 1]);  // +inf before the first tile
+        if (e < 2 ? dead0 : dead1) x[n][e] = -INFINITY;
+      }
+      move |= fmaxf(fmaxf(x[n][0], x[n][1]), fmaxf(x[n][2], x[n][3])) > kMoveThreshold;
+    }
+    if (__any_sync(0xFFFFFFFFu, move)) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        float alpha[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float mx = fmaxf(dead0 ? -INFINITY : s[n][h] * sl2, dead1 ? -INFINITY : s[n][2 + h] * sl2);
+          mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 4));
+          mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 8));
+          mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 16));
+          const float m_new = fmaxf(m_ref[n][h], mx);  // finite: every tile holds at least one live key
+          alpha[h] = ex2_approx(m_ref[n][h] - m_new);  // first tile: exp2(-inf) = 0
+          m_ref[n][h] = m_new;
+          l_run[n][h] *= alpha[h];
+        }
+#pragma unroll
+        for (int m = 0; m < D / 16; ++m) {
+          oacc[n][m][0] *= alpha[0];
+          oacc[n][m][1] *= alpha[1];
+          oacc[n][m][2] *= alpha[0];
+          oacc[n][m][3] *= alpha[1];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          x[n][e] = fmaf(s[n][e], sl2, -m_ref[n][e & 1]);
+          if (e < 2 ? dead0 : dead1) x[n][e] = -INFINITY;
+        }
       }
     }
-    float alpha[2];
+    uint32_t pb[NT][2];  // P^T fragments (B operand): keys 2 tq, 2 tq + 1 (+ 8) of head g0
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      float mx = fmaxf(fmaxf(sacc[0][2 * r], sacc[0][2 * r + 1]), fmaxf(sacc[1][2 * r], sacc[1][2 * r + 1]));
-      mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
-      mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
-      const float m_new = fmaxf(m_run[r], mx);  // finite: every tile holds at least one live key
-      alpha[r] = ex2_approx(m_run[r] - m_new);  // first tile: exp2(-inf) = 0
-      m_run[r] = m_new;
-      float sum = 0.f;
+    for (int n = 0; n < NT; ++n) {
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
-        const float p0 = ex2_approx(sacc[nb][2 * r] - m_new);
-        const float p1 = ex2_approx(sacc[nb][2 * r + 1] - m_new);
-        sacc[nb][2 * r] = p0;
-        sacc[nb][2 * r + 1] = p1;
-        sum += p0 + p1;
-      }
-      l_run[r] = l_run[r] * alpha[r] + sum;
+      for (int e = 0; e < 4; ++e) x[n][e] = ex2_approx(x[n][e]);
+      l_run[n][0] += x[n][0] + x[n][2];
+      l_run[n][1] += x[n][1] + x[n][3];
+      pb[n][0] = movmatrix_trans(pack2<BF16>(x[n][0], x[n][1]));
+      pb[n][1] = movmatrix_trans(pack2<BF16>(x[n][2], x[n][3]));
     }
-    if (__any_sync(0xFFFFFFFFu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-#pragma unroll
-      for (int n = 0; n < D / 8; ++n) {
-        oacc[n][0] *= alpha[0];
-        oacc[n][1] *= alpha[0];
-        oacc[n][2] *= alpha[1];
-        oacc[n][3] *= alpha[1];
-      }
-    }
-    uint32_t pa[4];
-    pa[0] = pack2<BF16>(sacc[0][0], sacc[0][1]);
-    pa[1] = pack2<BF16>(sacc[0][2], sacc[0][3]);
-    pa[2] = pack2<BF16>(sacc[1][0], sacc[1][1]);
-    pa[3] = pack2<BF16>(sacc[1][2], sacc[1][3]);
 
-    // ---- O[16 heads x D] += P V ----
+    // ---- O^T[D x 8 heads] += V^T P^T ----
     if constexpr (Q8) {
-      // B fragments pair two keys per register: lane (g0, tq) reads, for keys 2 tq, 2 tq + 1, 2 tq + 8, 2 tq + 9, the
-      // four bytes at dimensions 4 g0 .. 4 g0 + 3 of every block, interleaves the rows pairwise and converts.
-      // Output tile 4 blk + j then holds, in column c, dimension 32 blk + 4 c + j (see q8_dim below).
-      const uint8_t* rv = raw_k + kQTileBytes + (2 * tq) * kQRowBytes + 4 * g0;
+      // A fragments pair two keys per register: lane (g0, tq) reads, for keys 2 tq, 2 tq + 1, 2 tq + 8, 2 tq + 9, the
+      // four bytes at dimensions 4 g0 .. 4 g0 + 3 of every block, interleaves the rows pairwise and converts.  Row r of
+      // 16-row tile 2 blk + j is then dimension 32 blk + 4 (r % 8) + 2 j + r / 8.
+      const uint8_t* rv = raw_k + kTileBytes + (2 * tq) * kQRowBytes;
       // The copy zero-fills whole 16-byte pieces beyond the chunk, so the first row past the end can hold a few
       // real cache bytes, a scale among them: rows past the end get scale 0 (their weights are 0, and 0 * 0 = 0
       // whatever the cache holds there).
-      uint32_t row_ok[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) row_ok[r] = (key0 + 2 * tq + (r & 1) + 8 * (r >> 1) < c1) ? 0xFFFFu : 0u;
+      uint32_t ok01 = 0xFFFFFFFFu, ok23 = 0xFFFFFFFFu;
+      if (partial) {
+        const int left = c1 - key0 - 2 * tq;
+        ok01 = (left > 0 ? 0xFFFFu : 0u) | (left > 1 ? 0xFFFF0000u : 0u);
+        ok23 = (left > 8 ? 0xFFFFu : 0u) | (left > 9 ? 0xFFFF0000u : 0u);
+      }
 #pragma unroll
       for (int blk = 0; blk < D / 32; ++blk) {
-        uint32_t x[4], dsc[4];
+        uint32_t w[4], dsc[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const uint8_t* bp = rv + ((r & 1) + 8 * (r >> 1)) * kQRowBytes + blk * 34;
-          dsc[r] = *reinterpret_cast<const uint16_t*>(bp - 4 * g0) & row_ok[r];
-          uint32_t w;
-          if (blk & 1) {  // 34 blk + 2 is a multiple of 4 for odd blocks
-            w = *reinterpret_cast<const uint32_t*>(bp + 2);
-          } else {
-            w = static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(bp + 2)) |
-                (static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(bp + 4)) << 16);
-          }
-          x[r] = w ^ 0x80808080u;
+          dsc[r] = *reinterpret_cast<const uint16_t*>(bp);
+          w[r] = ld_q8_word(bp + 2 + 4 * g0, (blk & 1) != 0) ^ 0x80808080u;
         }
-        const Q8Scale<BF16> d01 = q8_scale<BF16>(dsc[0], dsc[1]);
-        const Q8Scale<BF16> d23 = q8_scale<BF16>(dsc[2], dsc[3]);
-        const uint32_t lo01 = __byte_perm(x[0], x[1], 0x5140), hi01 = __byte_perm(x[0], x[1], 0x7362);
-        const uint32_t lo23 = __byte_perm(x[2], x[3], 0x5140), hi23 = __byte_perm(x[2], x[3], 0x7362);
-        mma_16816<BF16>(oacc[4 * blk + 0], pa, q8_pair<BF16, 0, 1>(lo01, d01), q8_pair<BF16, 0, 1>(lo23, d23));
-        mma_16816<BF16>(oacc[4 * blk + 1], pa, q8_pair<BF16, 2, 3>(lo01, d01), q8_pair<BF16, 2, 3>(lo23, d23));
-        mma_16816<BF16>(oacc[4 * blk + 2], pa, q8_pair<BF16, 0, 1>(hi01, d01), q8_pair<BF16, 0, 1>(hi23, d23));
-        mma_16816<BF16>(oacc[4 * blk + 3], pa, q8_pair<BF16, 2, 3>(hi01, d01), q8_pair<BF16, 2, 3>(hi23, d23));
+        const Q8Scale<BF16> d01 = q8_scale_pair<BF16>((dsc[0] | (dsc[1] << 16)) & ok01);
+        const Q8Scale<BF16> d23 = q8_scale_pair<BF16>((dsc[2] | (dsc[3] << 16)) & ok23);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t e01 = __byte_perm(w[0], w[1], j ? 0x7362 : 0x5140), e23 = __byte_perm(w[2], w[3], j ? 0x7362 : 0x5140);
+          const uint32_t vf[4] = {q8_pair<BF16, 0, 1>(e01, d01), q8_pair<BF16, 2, 3>(e01, d01),
+                                  q8_pair<BF16, 0, 1>(e23, d23), q8_pair<BF16, 2, 3>(e23, d23)};
+#pragma unroll
+          for (int n = 0; n < NT; ++n) mma_16816<BF16>(oacc[n][2 * blk + j], vf, pb[n][0], pb[n][1]);
+        }
       }
     } else {
+      const uint32_t sv = sk + kTileBytes;
 #pragma unroll
-      for (int dn = 0; dn < D / 16; ++dn) {
-        uint32_t r0, r1, r2, r3;
-        const int key = (lm_mi & 1) * 8 + lm_r;
-        const int chunk = 2 * dn + (lm_mi >> 1);
-        ldmatrix_x4_trans(sv + swz<D>(key, chunk), r0, r1, r2, r3);
-        mma_16816<BF16>(oacc[2 * dn], pa, r0, r1);
-        mma_16816<BF16>(oacc[2 * dn + 1], pa, r2, r3);
+      for (int m = 0; m < D / 16; ++m) {
+        uint32_t vf[4];
+        ldmatrix_x4_trans(sv + swz<D>((lm_mi >> 1) * 8 + lm_r, 2 * m + (lm_mi & 1)), vf[0], vf[1], vf[2], vf[3]);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma_16816<BF16>(oacc[n][m], vf, pb[n][0], pb[n][1]);
       }
     }
   }
   cp_async_wait<0>();
 
-  // ---- row sums across the 4 lanes of a row ----
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    l_run[r] += __shfl_xor_sync(0xFFFFFFFFu, l_run[r], 1);
-    l_run[r] += __shfl_xor_sync(0xFFFFFFFFu, l_run[r], 2);
-  }
-
   // ---- merge the warps through shared memory (reusing the ring buffers) ----
+  const int group = a.group;
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      l_run[n][h] += __shfl_xor_sync(0xFFFFFFFFu, l_run[n][h], 4);
+      l_run[n][h] += __shfl_xor_sync(0xFFFFFFFFu, l_run[n][h], 8);
+      l_run[n][h] += __shfl_xor_sync(0xFFFFFFFFu, l_run[n][h], 16);
+    }
   __syncthreads();
-  float* mo = reinterpret_cast<float*>(wsm);             // [16][D]
-  float* mml = reinterpret_cast<float*>(wsm) + 16 * D;   // [16][2]
+  constexpr int kRow = D + 4;  // floats per head: the four lanes of a row fall into different banks
+  float* mo = reinterpret_cast<float*>(wsm);
+  float2* wml = reinterpret_cast<float2*>(smem + L::kRingBytes);                       // [kWarps][8 NT] (max, sum) per warp
+  float* pbuf = reinterpret_cast<float*>(smem + L::kRingBytes + L::kWmlBytes);         // [n_parts][slice] this block's slice
+  float2* pml = reinterpret_cast<float2*>(smem + L::kRingBytes + L::kWmlBytes + L::kPartBytes);  // [n_parts][group]
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int g = g0 + 8 * r;
-    if (g < a.group) {
+  for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int n = 0; n < D / 8; ++n) {
-        if constexpr (Q8) {
-          // column c of output tile 4 blk + j is dimension 32 blk + 4 c + j; this lane holds columns 2 tq, 2 tq + 1
-          const int d0 = 32 * (n >> 2) + 8 * tq + (n & 3);
-          mo[g * D + d0] = oacc[n][2 * r];
-          mo[g * D + d0 + 4] = oacc[n][2 * r + 1];
-        } else {
-          *reinterpret_cast<float2*>(&mo[g * D + n * 8 + tq * 2]) = make_float2(oacc[n][2 * r], oacc[n][2 * r + 1]);
+    for (int h = 0; h < 2; ++h) {
+      const int g = 8 * n + 2 * tq + h;
+      if (g < group) {
+#pragma unroll
+        for (int m = 0; m < D / 16; ++m) {
+          if constexpr (Q8) {
+            *reinterpret_cast<float2*>(&mo[g * kRow + 32 * (m >> 1) + 4 * g0 + 2 * (m & 1)]) = make_float2(oacc[n][m][h], oacc[n][m][2 + h]);
+          } else {
+            mo[g * kRow + 16 * m + g0] = oacc[n][m][h];
+            mo[g * kRow + 16 * m + 8 + g0] = oacc[n][m][2 + h];
+          }
         }
-      }
-      if (tq == 0) {
-        mml[g * 2] = m_run[r];
-        mml[g * 2 + 1] = l_run[r];
+        if (g0 == 0) wml[warp * 8 * NT + g] = make_float2(m_ref[n][h], l_run[n][h]);
       }
     }
-  }
   __syncthreads();
-  for (int idx = tid; idx < a.group * D; idx += kWarps * 32) {
-    const int g = idx / D;
-    const int d = idx % D;
-    float mw[kWarps];
+  const bool exchange = clustered && n_parts > 1;
+  const int slice = exchange ? group * D / n_parts : group * D;  // output values per block (a multiple of 4)
+  if (exchange) {
+    cluster_wait();  // every block of the cluster has started
+    // (max, sum) of this block to every block of the cluster
+    for (int t = tid; t < n_parts * group; t += kWarps * 32) {
+      const int r = t / group, g = t - r * group;
+      float M = -INFINITY, l = 0.f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) M = fmaxf(M, wml[w * 8 * NT + g].x);
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const float2 ml = wml[w * 8 * NT + g];
+        l += (ml.x == -INFINITY) ? 0.f : ex2_approx(ml.x - M) * ml.y;
+      }
+      st_cluster_v2(cluster_map(smem_u32(&pml[part * group + g]), r), M, l);
+    }
+  }
+  for (int e4 = tid; e4 < group * (D / 4); e4 += kWarps * 32) {
+    const int g = e4 / (D / 4), d = (e4 % (D / 4)) * 4;
+    float2 ml[kWarps];
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      mw[w] = reinterpret_cast<const float*>(smem + w * kWarpBytes)[16 * D + g * 2];
-      M = fmaxf(M, mw[w]);
+      ml[w] = wml[w * 8 * NT + g];
+      M = fmaxf(M, ml[w].x);
     }
-    float o = 0.f, l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float* wf = reinterpret_cast<const float*>(smem + w * kWarpBytes);
-      const float sc = (mw[w] == -INFINITY) ? 0.f : ex2_approx(mw[w] - M);
-      o += sc * wf[g * D + d];
-      l += sc * wf[16 * D + g * 2 + 1];
+      const float sc = (ml[w].x == -INFINITY) ? 0.f : ex2_approx(ml[w].x - M);
+      const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem + w * kWarpBytes) + g * kRow + d);
+      o.x += sc * x.x;
+      o.y += sc * x.y;
+      o.z += sc * x.z;
+      o.w += sc * x.w;
+      l += sc * ml[w].y;
     }
-    const int h = kvh * a.group + g;
-    const size_t pidx = (static_cast<size_t>(b) * a.n_heads + h) * a.n_split + split;
-    a.part_o[pidx * D + d] = o;
-    if (d == 0) {
-      a.part_ml[pidx * 2] = M;
-      a.part_ml[pidx * 2 + 1] = l;
+    const int h = kvh * group + g;
+    if (exchange) {
+      // the block whose slice holds these four values gets them
+      const int e = g * D + d, r = e / slice;
+      st_cluster_v4(cluster_map(smem_u32(&pbuf[part * slice + (e - r * slice)]), r), o);
+    } else if (clustered) {
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      uint8_t* op = reinterpret_cast<uint8_t*>(a.out) +
+                    2 * (static_cast<size_t>(b) * a.out_stride[0] + static_cast<size_t>(h) * a.out_stride[1] + d);
+      *reinterpret_cast<uint2*>(op) = make_uint2(pack2<BF16>(o.x * inv, o.y * inv), pack2<BF16>(o.z * inv, o.w * inv));
+    } else {
+      const size_t pidx = (static_cast<size_t>(b) * a.n_heads + h) * n_parts + part;
+      *reinterpret_cast<float4*>(a.part_o + pidx * D + d) = o;
+      if (d == 0) *reinterpret_cast<float2*>(a.part_ml + pidx * 2) = make_float2(M, l);
     }
+  }
+  if (!exchange) return;
+  // ---- merge the cluster's blocks: each finishes its slice of the output ----
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  for (int t = 2 * tid; t < slice; t += 2 * kWarps * 32) {
+    const int e = part * slice + t, g = e / D, d = e % D;
+    float M = -INFINITY, l = 0.f, o0 = 0.f, o1 = 0.f;
+    for (int p = 0; p < n_parts; ++p) M = fmaxf(M, pml[p * group + g].x);
+    for (int p = 0; p < n_parts; ++p) {
+      const float2 ml = pml[p * group + g];
+      const float sc = (ml.x == -INFINITY) ? 0.f : ex2_approx(ml.x - M);
+      const float2 x = *reinterpret_cast<const float2*>(&pbuf[p * slice + t]);
+      o0 += sc * x.x;
+      o1 += sc * x.y;
+      l += sc * ml.y;
+    }
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    uint8_t* op = reinterpret_cast<uint8_t*>(a.out) + 2 * (static_cast<size_t>(b) * a.out_stride[0] +
+                                                           static_cast<size_t>(kvh * group + g) * a.out_stride[1] + d);
+    *reinterpret_cast<uint32_t*>(op) = pack2<BF16>(o0 * inv, o1 * inv);
   }
 }
 
@@ -451,6 +614,8 @@ __global__ void __launch_bounds__(D) decode_combine_kernel(const DecodeArgs a) {
   const int h = blockIdx.x;
   const int b = blockIdx.y;
   const int d = threadIdx.x;
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int len = min(a.lens[b], a.max_len);
   const int ns = (len + a.chunk - 1) / a.chunk;
   const size_t p0 = (static_cast<size_t>(b) * a.n_heads + h) * a.n_split;
@@ -489,31 +654,40 @@ __global__ void __launch_bounds__(D) decode_combine_kernel(const DecodeArgs a) {
   else *reinterpret_cast<__half*>(op) = __float2half_rn(r);
 }
 
-template <int D, bool BF16, bool Q8, bool Paged>
-cudaError_t launch_paged(const DecodeArgs& a, cudaStream_t stream) {
-  constexpr int kRaw = Q8 ? kTileKeys * (D / 32) * 34 : kTileKeys * D * 2;
-  constexpr int smem = kWarps * (Q8 ? MINFER_ATTN_Q8_STAGES : kStages) * 2 * kRaw;
-  static_assert(smem / kWarps >= 16 * D * 4 + 128, "the per-warp region also holds the fp32 merge buffer");
-  static std::atomic<bool> attr_done[64] = {};  // set-once flags; the attribute call itself is idempotent
+template <int D, bool BF16, bool Q8, bool Paged, int NT>
+cudaError_t launch_heads(const DecodeArgs& a, cudaStream_t stream) {
+  auto* kernel = decode_kernel<D, BF16, Q8, Paged, NT>;
+  constexpr int smem = Layout<D, Q8, NT>::kBytes;
+  static std::atomic<bool> attr_done[64] = {};  // set-once flags; the attribute calls themselves are idempotent
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 64 && !attr_done[dev].load(std::memory_order_acquire)) {
-    e = cudaFuncSetAttribute(decode_split_kernel<D, BF16, Q8, Paged>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (dev >= 64 || !attr_done[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    attr_done[dev].store(true, std::memory_order_release);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) attr_done[dev].store(true, std::memory_order_release);
   }
-  dim3 grid(a.n_split, a.n_kv_heads, a.batch);
-  decode_split_kernel<D, BF16, Q8, Paged><<<grid, kWarps * 32, smem, stream>>>(a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  decode_combine_kernel<D, BF16><<<dim3(a.n_heads, a.batch), D, 0, stream>>>(a);
-  return cudaGetLastError();
+  const bool clustered = a.part_o == nullptr;
+  LaunchAttrs at(stream);
+  at.cfg.gridDim = dim3(a.n_split, a.n_kv_heads, a.batch);
+  at.cfg.blockDim = dim3(kWarps * 32);
+  at.cfg.dynamicSmemBytes = smem;
+  if (clustered && a.n_split > 1) at.cluster(a.n_split);
+  e = cudaLaunchKernelEx(&at.cfg, kernel, a);
+  if (e != cudaSuccess || clustered) return e;
+  LaunchAttrs ac(stream);
+  ac.cfg.gridDim = dim3(a.n_heads, a.batch);
+  ac.cfg.blockDim = dim3(D);
+  return cudaLaunchKernelEx(&ac.cfg, decode_combine_kernel<D, BF16>, a);
 }
 
 template <int D, bool BF16, bool Q8>
 cudaError_t launch_one(const DecodeArgs& a, cudaStream_t stream) {
-  return a.block_table != nullptr ? launch_paged<D, BF16, Q8, true>(a, stream) : launch_paged<D, BF16, Q8, false>(a, stream);
+  if (a.group <= 8)
+    return a.block_table != nullptr ? launch_heads<D, BF16, Q8, true, 1>(a, stream) : launch_heads<D, BF16, Q8, false, 1>(a, stream);
+  return a.block_table != nullptr ? launch_heads<D, BF16, Q8, true, 2>(a, stream) : launch_heads<D, BF16, Q8, false, 2>(a, stream);
 }
 
 }  // namespace

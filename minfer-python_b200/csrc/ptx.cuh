@@ -350,6 +350,33 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
 }
 
 // ---------------------------------------------------------------------------
+// dependent launches and clusters
+// ---------------------------------------------------------------------------
+// Kernels of this library are launched with programmatic stream serialisation: a kernel's blocks may be placed while
+// the kernel before it still runs.  Each lets its own successor do the same at once, and touches no memory that
+// another kernel may write or read before grid_dependency_wait() - which returns when every earlier kernel of
+// the stream has completed and its writes are visible.  (Both are no-ops in an ordinary launch.)
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// barrier over all threads of the cluster, in two halves (release / acquire: shared-memory writes before the arrive are
+// visible to the cluster's other blocks after the wait)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// address of the same shared-memory location in block `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void st_cluster_v2(uint32_t addr, float x, float y) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // legacy warp-level pieces used by the HBM-bound decode kernel
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc, bool pred) {
@@ -373,6 +400,13 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t saddr, uint32_t& r0, 
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                : "r"(saddr));
+}
+
+// transpose of an 8x8 matrix of 16-bit values held one row per four lanes
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
+  uint32_t r;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
+  return r;
 }
 
 // D(16x8, f32) += A(16x16) * B(16x8), 16-bit inputs

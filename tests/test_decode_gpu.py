@@ -174,3 +174,34 @@ def test_random_shapes_against_the_oracle(kerns, seed):
         check_close_bf16_by_keys(got[live], want[live], lens[live].view(-1, 1, 1, 1), what)
     else:
         check_close(got[live], want[live], what)
+
+
+@pytest.mark.parametrize("B,Hkv,group,D,Lmax,dtype", [
+    (1, 1, 1, 64, 15, torch.float16), (1, 2, 16, 128, 1100, torch.bfloat16),   # one block; clusters of 16, two column tiles
+    (9, 2, 9, 64, 1024, torch.float16), (40, 2, 4, 128, 150, torch.float16),   # clusters of 8 and of 2
+    (150, 2, 8, 64, 300, torch.bfloat16),                                      # more pairs than one wave of blocks
+    (256, 1, 2, 128, 1300, torch.float16), (257, 1, 2, 128, 1300, torch.float16)])  # large, ordered by length and not
+def test_block_clusters_and_order_by_length(kerns, B, Hkv, group, D, Lmax, dtype):
+    """Every cluster size and both orders, with lengths at the edges of the 16-key tiles and of the shares of a
+    cluster's blocks (so that some blocks get nothing), empty sequences and equal lengths among them."""
+    g = torch.Generator().manual_seed(B + D)
+    H = Hkv * group
+    lens = torch.randint(0, Lmax + 1, (B,), generator=g, dtype=torch.int32)
+    edges = [Lmax, 0, 1, 16, 17, min(Lmax, 127), min(Lmax, 256), min(Lmax, 256)]
+    lens[:min(B, len(edges))] = torch.tensor(edges[:B], dtype=torch.int32)
+    q = torch.randn(B, H, 1, D, generator=g).to(dtype)
+    kc = torch.randn(B, Hkv, Lmax, D, generator=g).to(dtype)
+    vc = torch.randn(B, Hkv, Lmax, D, generator=g).to(dtype)
+    want = O.attention_f64(q, kc, vc, lens=lens)
+    for b in range(B):
+        kc[b, :, int(lens[b]):] = float("nan")
+        vc[b, :, int(lens[b]):] = float("nan")
+    got = run_decode(kerns, q, kc, vc, lens)
+    assert torch.count_nonzero(got[lens == 0]) == 0
+    live = lens > 0
+    if dtype == torch.bfloat16:
+        from _util import check_close_bf16_by_keys
+        check_close_bf16_by_keys(got[live], want[live], lens[live].view(-1, 1, 1, 1), f"B={B}")
+    else:
+        check_close(got[live], want[live], f"B={B} D={D}")
+    assert torch.equal(got, run_decode(kerns, q, kc, vc, lens))
