@@ -118,15 +118,12 @@ __device__ __forceinline__ void round16(float (&x)[8]) {
 #ifndef MINFER_ATTN_ROPE_MINBLOCKS
 #define MINFER_ATTN_ROPE_MINBLOCKS 4
 #endif
-// Loads staged in shared memory by asynchronous copies before the thread works through them (0: plain loads into
-// registers, four rows at a time).  Measured on the prefill-sized call (B=4, L=4096, 32/8 heads, D=128; interleaved /
-// two-halves / D=64 interleaved, us): registers 77.7 / 84.1 / 47.4; one buffer of 6 chunks 72.0 / 70.9 / 43.0 (8
-// chunks 74.1 / 70.4 / 43.2, 10 chunks 79.2 / 72.2 / 44.7); two buffers of 4 chunks, the next batch in flight while
-// this one is worked on, 67.4 / 78.0 / 41.4 (of 2 chunks 70.0 / 76.0 / 43.2).  The interleaved form therefore uses two
-// buffers of four rows, the two-halves form (two chunks per row, more registers) one buffer of three rows.
-#ifndef MINFER_ATTN_ROPE_STAGED
-#define MINFER_ATTN_ROPE_STAGED 1
-#endif
+// Loads staged in shared memory by asynchronous copies before the thread works through them.  Measured on the
+// prefill-sized call (B=4, L=4096, 32/8 heads, D=128; interleaved / two-halves / D=64 interleaved, us): loads into
+// registers 77.7 / 84.1 / 47.4; one buffer of 6 chunks 72.0 / 70.9 / 43.0 (8 chunks 74.1 / 70.4 / 43.2, 10 chunks 79.2 /
+// 72.2 / 44.7); two buffers of 4 chunks, the next batch in flight while this one is worked on, 67.4 / 78.0 / 41.4 (of 2
+// chunks 70.0 / 76.0 / 43.2).  The interleaved form therefore uses two buffers of four rows, the two-halves form (two
+// chunks per row, more registers) one buffer of three rows.  The first batch is issued before the position is known.
 #ifndef MINFER_ATTN_ROPE_SLICES
 #define MINFER_ATTN_ROPE_SLICES 4
 #endif
@@ -135,7 +132,6 @@ constexpr int kRopePairs = 256 / kRopeSlices;         // (token, chunk) pairs pe
 
 template <bool BF16, bool kNeox>
 __global__ void __launch_bounds__(kRopePairs * kRopeSlices, MINFER_ATTN_ROPE_MINBLOCKS) rope_append_kernel(const RopeArgs a) {
-  constexpr int kRopeRows = kNeox ? 2 : 4;           // rows a thread loads before it computes
   __shared__ __align__(16) float s_cs[kRopePairs][8];
   __shared__ __align__(16) float s_sn[kRopePairs][8];
   const int chunks = a.head_dim / 8;                 // 16-byte chunks per head row
@@ -167,6 +163,70 @@ __global__ void __launch_bounds__(kRopePairs * kRopeSlices, MINFER_ATTN_ROPE_MIN
   }
   const int b = static_cast<int>(token / static_cast<unsigned>(a.seq));
   const int l = static_cast<int>(token - static_cast<unsigned>(b) * static_cast<unsigned>(a.seq));
+  grid_launch_dependents();
+  grid_dependency_wait();
+
+  const size_t co = static_cast<size_t>(c) * 16, co2 = static_cast<size_t>(c2 < 0 ? 0 : c2) * 16;
+  // The rows of this token - its query heads, then its k heads, then its v heads - are dealt out over
+  // gridDim.y slices, and a thread takes its rows four at a time, all loads first: a thread that walked
+  // every head alone, one dependent load at a time, left the memory system idle (decode-sized calls took
+  // tens of microseconds, prefill-sized ones reached 0.64 of the copy bandwidth).
+  // The row list is the same for every thread of the launch (the threads that share a Q8_0 block must
+  // meet in the same row at the same step); what differs per thread is which kinds of row it has work for.
+  const int n_q = a.q != nullptr ? a.n_heads : 0;
+  const int n_k = a.k != nullptr ? a.n_kv_heads : 0;
+  const int n_rows = n_q + n_k + ((a.v != nullptr && a.v_cache != nullptr) ? a.n_kv_heads : 0);
+  const uint8_t* q_base = reinterpret_cast<const uint8_t*>(a.q) + 2 * (static_cast<size_t>(b) * a.q_stride[0] + static_cast<size_t>(l) * a.q_stride[1]);
+  const uint8_t* k_base = reinterpret_cast<const uint8_t*>(a.k) + 2 * (static_cast<size_t>(b) * a.kv_stride[0] + static_cast<size_t>(l) * a.kv_stride[1]);
+  const uint8_t* v_base = reinterpret_cast<const uint8_t*>(a.v) + 2 * (static_cast<size_t>(b) * a.kv_stride[0] + static_cast<size_t>(l) * a.kv_stride[1]);
+  // source row of combined row index r (kind 0 = q, 1 = k, 2 = v) and its head
+  auto row_of = [&](int r, int& kind, int& h) -> const uint8_t* {
+    if (r < n_q) {
+      kind = 0;
+      h = r;
+      return q_base + 2 * static_cast<size_t>(h) * a.q_stride[2];
+    }
+    if (r < n_q + n_k) {
+      kind = 1;
+      h = r - n_q;
+      return k_base + 2 * static_cast<size_t>(h) * a.kv_stride[2];
+    }
+    kind = 2;
+    h = r - n_q - n_k;
+    return v_base + 2 * static_cast<size_t>(h) * a.kv_stride[2];
+  };
+  // The first batch is on its way before the position, the block table and the angles are known: what is read does not
+  // depend on them (a row whose position turns out to lie outside the cache is read and dropped).
+  const bool to_cache = a.k_cache != nullptr;  // the call appends (as opposed to rotating k in place)
+  auto loaded = [&](int kd) { return kd == 0 ? rotate : (kd == 1 ? to_cache || rotate : true); };
+  const int n_slices = static_cast<int>(gridDim.y) * kRopeSlices;
+  // Loads through shared memory: a thread issues the 16-byte asynchronous copies of up to kStageRows of its rows
+  // (cp.async, no registers held while they fly), waits for its own copies and then works through the rows.
+  constexpr int kNC = kNeox ? 2 : 1;                                    // chunks per row and thread
+  constexpr int kStageRows = kNeox ? 3 : 4;                             // rows per batch
+  constexpr int kBufs = kNeox ? 1 : 2;                                  // 2: the next batch flies while this one is worked on
+  constexpr int kBatch = kStageRows * kNC * kRopePairs * kRopeSlices;   // uint4 per buffer
+  __shared__ __align__(16) uint4 s_rows[kBufs * kBatch];
+  const int tid = static_cast<int>(threadIdx.x);
+  const int step = kStageRows * n_slices;
+  auto issue = [&](int r0, int buf) {
+#pragma unroll
+    for (int j = 0; j < kStageRows; ++j) {
+      const int r = r0 + j * n_slices;
+      if (r < n_rows) {
+        int kd, h;
+        const uint8_t* srcp = row_of(r, kd, h);
+        if (loaded(kd)) {
+          cp_async_16(&s_rows[buf * kBatch + (j * kNC) * 256 + tid], srcp + co, true);
+          if (kNeox && c2 >= 0) cp_async_16(&s_rows[buf * kBatch + (j * kNC + kNC - 1) * 256 + tid], srcp + co2, true);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  const int first = static_cast<int>(blockIdx.y) * kRopeSlices + slice_in;
+  if (valid && first < n_rows) issue(first, 0);
+
   const int pos = (a.start ? a.start[b] : a.start_pos) + l;
   // where the row of position `pos` starts inside a cache, in units of the cache strides, head offset excluded:
   // contiguous [batch][head][row] caches, or a pool of pages reached through the block table
@@ -198,7 +258,6 @@ __global__ void __launch_bounds__(kRopePairs * kRopeSlices, MINFER_ATTN_ROPE_MIN
     cb = static_cast<size_t>(page);
     crow = pos % a.page_size;
   }
-  const bool to_cache = a.k_cache != nullptr;  // the call appends (as opposed to rotating k in place)
 
   float cs[8], sn[8];
   {
@@ -232,38 +291,9 @@ __global__ void __launch_bounds__(kRopePairs * kRopeSlices, MINFER_ATTN_ROPE_MIN
 
   const int q_row_bytes = (a.head_dim / 32) * 34;  // a Q8_0 cache row
 
-  const size_t co = static_cast<size_t>(c) * 16, co2 = static_cast<size_t>(c2 < 0 ? 0 : c2) * 16;
-  // The rows of this token - its query heads, then its k heads, then its v heads - are dealt out over
-  // gridDim.y slices, and a thread takes its rows four at a time, all loads first: a thread that walked
-  // every head alone, one dependent load at a time, left the memory system idle (decode-sized calls took
-  // tens of microseconds, prefill-sized ones reached 0.64 of the copy bandwidth).
-  // The row list is the same for every thread of the launch (the threads that share a Q8_0 block must
-  // meet in the same row at the same step); what differs per thread is which kinds of row it has work for.
   const bool do_q = rotate;
   const bool do_k = to_cache ? cache_ok : rotate;
   const bool do_v = cache_ok;
-  const int n_q = a.q != nullptr ? a.n_heads : 0;
-  const int n_k = a.k != nullptr ? a.n_kv_heads : 0;
-  const int n_rows = n_q + n_k + ((a.v != nullptr && a.v_cache != nullptr) ? a.n_kv_heads : 0);
-  const uint8_t* q_base = reinterpret_cast<const uint8_t*>(a.q) + 2 * (static_cast<size_t>(b) * a.q_stride[0] + static_cast<size_t>(l) * a.q_stride[1]);
-  const uint8_t* k_base = reinterpret_cast<const uint8_t*>(a.k) + 2 * (static_cast<size_t>(b) * a.kv_stride[0] + static_cast<size_t>(l) * a.kv_stride[1]);
-  const uint8_t* v_base = reinterpret_cast<const uint8_t*>(a.v) + 2 * (static_cast<size_t>(b) * a.kv_stride[0] + static_cast<size_t>(l) * a.kv_stride[1]);
-  // source row of combined row index r (kind 0 = q, 1 = k, 2 = v) and its head
-  auto row_of = [&](int r, int& kind, int& h) -> const uint8_t* {
-    if (r < n_q) {
-      kind = 0;
-      h = r;
-      return q_base + 2 * static_cast<size_t>(h) * a.q_stride[2];
-    }
-    if (r < n_q + n_k) {
-      kind = 1;
-      h = r - n_q;
-      return k_base + 2 * static_cast<size_t>(h) * a.kv_stride[2];
-    }
-    kind = 2;
-    h = r - n_q - n_k;
-    return v_base + 2 * static_cast<size_t>(h) * a.kv_stride[2];
-  };
   // one row of the token: rotate (q, k) or copy (v) this thread's chunk(s) and store them
   auto process = [&](int kd, int h, const uint8_t* srcp, const uint4& xa_, const uint4& xb_) {
       if (kd == 2) {  // v: copied into the cache
@@ -326,42 +356,14 @@ __global__ void __launch_bounds__(kRopePairs * kRopeSlices, MINFER_ATTN_ROPE_MIN
       if (rotate || drow != srcp) *reinterpret_cast<uint4*>(drow + co) = pack8<BF16>(ox);
       if (rotate && kNeox) *reinterpret_cast<uint4*>(drow + co2) = pack8<BF16>(oy);
   };
-  const int n_slices = static_cast<int>(gridDim.y) * kRopeSlices;
   auto wanted = [&](int kd) { return kd == 0 ? do_q : (kd == 1 ? do_k : do_v); };
-#if MINFER_ATTN_ROPE_STAGED
-  // Loads through shared memory: a thread issues the 16-byte asynchronous copies of up to kStageRows of its rows
-  // (cp.async, no registers held while they fly), waits for its own copies and then works through the rows.
-  constexpr int kNC = kNeox ? 2 : 1;                                    // chunks per row and thread
-  constexpr int kStageRows = kNeox ? 3 : 4;                             // rows per batch
-  constexpr int kBufs = kNeox ? 1 : 2;                                  // 2: the next batch flies while this one is worked on
-  constexpr int kBatch = kStageRows * kNC * kRopePairs * kRopeSlices;   // uint4 per buffer
-  __shared__ __align__(16) uint4 s_rows[kBufs * kBatch];
-  const int tid = static_cast<int>(threadIdx.x);
-  const int step = kStageRows * n_slices;
-  auto issue = [&](int r0, int buf) {
-#pragma unroll
-    for (int j = 0; j < kStageRows; ++j) {
-      const int r = r0 + j * n_slices;
-      if (r < n_rows) {
-        int kd, h;
-        const uint8_t* srcp = row_of(r, kd, h);
-        if (wanted(kd)) {
-          cp_async_16(&s_rows[buf * kBatch + (j * kNC) * 256 + tid], srcp + co, true);
-          if (kNeox && c2 >= 0) cp_async_16(&s_rows[buf * kBatch + (j * kNC + kNC - 1) * 256 + tid], srcp + co2, true);
-        }
-      }
-    }
-    cp_async_commit();
-  };
-  const int first = static_cast<int>(blockIdx.y) * kRopeSlices + slice_in;
-  if (kBufs == 2 && first < n_rows) issue(first, 0);
   int buf = 0;
   for (int r0 = first; r0 < n_rows; r0 += step, buf ^= (kBufs - 1)) {
     if constexpr (kBufs == 2) {
       issue(r0 + step, buf ^ 1);     // (an empty group when there is no next batch)
       cp_async_wait<1>();
     } else {
-      issue(r0, 0);
+      if (r0 != first) issue(r0, 0);
       cp_async_wait<0>();
     }
 #pragma unroll
@@ -376,31 +378,6 @@ __global__ void __launch_bounds__(kRopePairs * kRopeSlices, MINFER_ATTN_ROPE_MIN
       process(kd, h, srcp, xa_, xb_);
     }
   }
-#else
-  for (int r0 = static_cast<int>(blockIdx.y) * kRopeSlices + slice_in; r0 < n_rows; r0 += kRopeRows * n_slices) {
-    const uint8_t* src[kRopeRows];
-    int kind[kRopeRows], hh[kRopeRows];
-    uint4 xa[kRopeRows], xb[kRopeRows];
-#pragma unroll
-    for (int j = 0; j < kRopeRows; ++j) {
-      const int r = r0 + j * n_slices;
-      kind[j] = -1;
-      if (r < n_rows) {
-        src[j] = row_of(r, kind[j], hh[j]);
-        if (!wanted(kind[j])) kind[j] = -1;  // nothing to do for this row
-      }
-      if (kind[j] >= 0) {
-        xa[j] = *reinterpret_cast<const uint4*>(src[j] + co);
-        if (c2 >= 0) xb[j] = *reinterpret_cast<const uint4*>(src[j] + co2);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kRopeRows; ++j) {
-      if (kind[j] < 0) continue;
-      process(kind[j], hh[j], src[j], xa[j], xb[j]);
-    }
-  }
-#endif
 }
 
 }  // namespace
@@ -430,25 +407,25 @@ cudaError_t launch_rope_append(const RopeArgs& a_in, bool bf16, bool neox, cudaS
   const int work_chunks = neox ? chunks - a.rotary_dim / 16 : chunks;
   const long long pairs = static_cast<long long>(a.batch) * a.seq * work_chunks;
   // A block serves 64 (token, chunk) pairs with four threads each, one per slice of the token's rows (query heads +
-  // k heads + v heads).  Small calls get further slices over gridDim.y, down to one row per thread, so that the
-  // grid still covers the GPU; large ones keep at least four rows per thread (all loads of a step in flight).
+  // k heads + v heads).  Calls that do not fill the GPU get further slices over gridDim.y, down to one row per thread,
+  // but no more than one wave of blocks (four per SM): a block's life is a chain of latencies (position, angles, load,
+  // store), so a second wave costs more than the rows it takes off the threads of the first.  Measured (us at 148 / 592 /
+  // 1184 / 3552 blocks): 8 x 512 tokens, 32/8 heads, D=64 12.0 / 12.1 / 13.3 / 17.7; 1000 tokens, D=128 11.0 / 8.1 / 9.0 / 14.6
+  // (two halves 15.4 / 8.5 / 9.6 / 10.4); 64 tokens 3.7 / 3.4 / 3.4 / 3.4.
+  constexpr long long kWave = 4 * 148;
   const int n_rows = (a.q != nullptr ? a.n_heads : 0) + (a.k != nullptr ? a.n_kv_heads : 0) +
                      (a.v != nullptr && a.v_cache != nullptr ? a.n_kv_heads : 0);
   if (pairs > 0x7FFFFFFFll - kRopePairs) return cudaErrorInvalidValue;  // the kernel indexes pairs in 32 bits
   const long long blocks_x = (pairs + kRopePairs - 1) / kRopePairs;
-  long long slices_y = (8 * 3 * 148 + blocks_x - 1) / blocks_x;
-  const long long max_slices = (pairs >= 65536 ? (n_rows + 3) / 4 : n_rows) / kRopeSlices;
+  long long slices_y = kWave / blocks_x;
+  const long long max_slices = n_rows / kRopeSlices;
   if (slices_y > max_slices) slices_y = max_slices;
   if (slices_y < 1) slices_y = 1;
-  const dim3 grid(static_cast<unsigned>(blocks_x), static_cast<unsigned>(slices_y));
-  if (bf16) {
-    if (neox) rope_append_kernel<true, true><<<grid, 256, 0, stream>>>(a);
-    else rope_append_kernel<true, false><<<grid, 256, 0, stream>>>(a);
-  } else {
-    if (neox) rope_append_kernel<false, true><<<grid, 256, 0, stream>>>(a);
-    else rope_append_kernel<false, false><<<grid, 256, 0, stream>>>(a);
-  }
-  return cudaGetLastError();
+  LaunchAttrs at(stream);
+  at.cfg.gridDim = dim3(static_cast<unsigned>(blocks_x), static_cast<unsigned>(slices_y));
+  at.cfg.blockDim = dim3(kRopePairs * kRopeSlices);
+  if (bf16) return neox ? cudaLaunchKernelEx(&at.cfg, rope_append_kernel<true, true>, a) : cudaLaunchKernelEx(&at.cfg, rope_append_kernel<true, false>, a);
+  return neox ? cudaLaunchKernelEx(&at.cfg, rope_append_kernel<false, true>, a) : cudaLaunchKernelEx(&at.cfg, rope_append_kernel<false, false>, a);
 }
 
 }  // namespace minfer_attn
