@@ -150,18 +150,19 @@ bool decode_is_large(int64_t pairs, int64_t max_len, int64_t row_bytes) { return
 
 // Blocks (one cluster) per (sequence, kv head) of a decode call, or 0: chunks, and a second kernel that merges them.
 // The lengths are on the device, so the rule knows the padded length only.
-//   A block costs about 4 us beside its keys (launch, the chain length -> keys -> scores, merge), and two fit an SM.
-//   While the caches hold little, a call is one such latency: as many blocks as one wave takes (296), no more.  Measured
-//   (us, 1 / 2 / 4 / 8 / 16 blocks): 1 sequence, 8 kv heads, 777 keys, D=128 7.5 / 6.5 / 5.4 / 4.7 / 4.7; 8 sequences of
-//   513-640, D=64 6.8 / 6.9 / 6.4 / 6.3 / 13.6; 8 of 2000-4096, D=128 32 / 23 / 19.7 / 21.2 / 33; 32 of 300 9.3 / 14.2 / 21 / ...
+//   A block costs about 4 us beside its keys (launch, the chain length -> keys -> scores, merge), and two fit an SM, four
+//   at head_dim 64.  While the caches hold little, a call is one such latency: as many blocks as one wave takes, no more.
+//   Measured (us, 1 / 2 / 4 / 8 / 16 blocks): 1 sequence, 8 kv heads, 777 keys, D=128 7.7 / 6.0 / 4.9 / 4.4 / 4.4; 8
+//   sequences of 513-640, D=64 6.8 / 6.6 / 6.1 / 5.8 / 11.5; 8 of 2000-4096, D=128 33 / 22.5 / 19.3 / 20.7 / 31; 32 of 300
+//   9.4 / 13.6 / 20 / 32 / 70.
 //   Large caches (worth 25 us of bandwidth and more) are taken in several waves, so that a batch of ragged lengths
 //   leaves no long tail (with the longest sequences first, see sequence_by_length): 64 sequences of 512-8192, 8 kv heads
-//   164 / 165 / 176 / 206; 24 of 100-6000 72 / 54.3 / 54.2 / 63; Q8_0, 64 of 512-8192 153 / 107 / 121 / 153.
+//   177 / 164 / 174 / 203; 24 of 100-6000 71 / 53.7 / 54.7 / 72; Q8_0, 64 of 512-8192 150 / 106 / 118 / 150.
 //   A handful of heads over a very long cache would leave most SMs without a block: chunks then.
 int decode_parts(int64_t batch, int64_t n_kv_heads, int64_t max_len, int64_t row_bytes) {
   const int64_t pairs = batch * n_kv_heads;
   if (pairs <= 4 && max_len >= 32768) return 0;
-  const int64_t limit = decode_is_large(pairs, max_len, row_bytes) ? 1024 : 2 * 148;
+  const int64_t limit = decode_is_large(pairs, max_len, row_bytes) ? 1024 : (row_bytes == 128 ? 4 : 2) * 148;
   int parts = 1;
   while (parts < 16 && pairs * parts * 2 <= limit && max_len >= 64 * parts * 2) parts *= 2;
   return parts;

@@ -74,7 +74,8 @@ struct Layout {
   static constexpr int kRingBytes = kWarps * kWarpBytes;
   static constexpr int kWmlBytes = kWarps * 8 * NT * 8;
   static constexpr int kPartBytes = 8 * NT * D * 4;
-  static constexpr int kBytes = kRingBytes + kWmlBytes + kPartBytes + kMaxParts * 8 * NT * 8;
+  static constexpr int kMlBytes = kMaxParts * 8 * NT * 8;
+  static constexpr int kBytes = kRingBytes + kWmlBytes + kPartBytes + kMlBytes + 16;  // + the arrival barrier, an abort flag
   static_assert(kWarpBytes >= 8 * NT * (D + 4) * 4, "the per-warp ring also holds the warp's partial output");
   static_assert(kRingBytes >= (kMaxRanked + 2) * 4, "the ranking by length borrows the ring");
 };
@@ -85,6 +86,14 @@ __device__ __noinline__ void report_bad_page(int32_t* status, int b, int slot, i
     status[1] = b;
     status[2] = slot;
     status[3] = page;
+  }
+}
+
+__device__ __noinline__ void report_wait(int32_t* status, int part) {
+  if (status != nullptr && atomicCAS(status, 0, kStatusWaitTimeout) == 0) {
+    status[1] = part;
+    status[2] = static_cast<int32_t>(blockIdx.z);
+    status[3] = 50;
   }
 }
 
@@ -198,8 +207,20 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
   const int part = blockIdx.x;       // which piece of the sequence
   const int n_parts = gridDim.x;
 
+  uint64_t* arrived = reinterpret_cast<uint64_t*>(smem + L::kBytes - 16);  // completes when all blocks' partial outputs are here
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(arrived + 1);
   grid_launch_dependents();
-  if (clustered && n_parts > 1) cluster_arrive();  // awaited before the first access to another block's shared memory
+  if (clustered && n_parts > 1) {
+    if (tid == 0) {
+      *abort_flag = 0;
+      mbar_init(arrived, 1);
+      mbar_fence_init();
+      // D / n_parts dimensions and the (max, sum) of every head, from every block
+      mbar_arrive_expect_tx(arrived, static_cast<uint32_t>(a.group * (D * 4 + n_parts * 8)));
+    }
+    __syncwarp();
+    cluster_arrive();  // awaited before the first access to another block's shared memory
+  }
   grid_dependency_wait();
 
   // ---- which sequence: in order, or the i-th longest (a.by_length: few enough sequences to rank them here) ----
@@ -507,8 +528,10 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
   constexpr int kRow = D + 4;  // floats per head: the four lanes of a row fall into different banks
   float* mo = reinterpret_cast<float*>(wsm);
   float2* wml = reinterpret_cast<float2*>(smem + L::kRingBytes);                       // [kWarps][8 NT] (max, sum) per warp
-  float* pbuf = reinterpret_cast<float*>(smem + L::kRingBytes + L::kWmlBytes);         // [n_parts][slice] this block's slice
+  float* pbuf = reinterpret_cast<float*>(smem + L::kRingBytes + L::kWmlBytes);         // [n_parts][group][dims]
   float2* pml = reinterpret_cast<float2*>(smem + L::kRingBytes + L::kWmlBytes + L::kPartBytes);  // [n_parts][group]
+  static_assert(D / 4 >= kMaxParts, "a head's four-dimension pieces cover the blocks of a cluster");
+  constexpr int kLogD = D == 128 ? 7 : 6;
 #pragma unroll
   for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -528,26 +551,15 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
       }
     }
   __syncthreads();
+  // Block r of the cluster finishes dimensions [r, r + 1) * D / n_parts of every head (n_parts is a power of two of at
+  // most D / 4).  All index arithmetic below is shifts: this is a chain of latencies, and a division by a runtime value is
+  // a tenth of it.
   const bool exchange = clustered && n_parts > 1;
-  const int slice = exchange ? group * D / n_parts : group * D;  // output values per block (a multiple of 4)
-  if (exchange) {
-    cluster_wait();  // every block of the cluster has started
-    // (max, sum) of this block to every block of the cluster
-    for (int t = tid; t < n_parts * group; t += kWarps * 32) {
-      const int r = t / group, g = t - r * group;
-      float M = -INFINITY, l = 0.f;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) M = fmaxf(M, wml[w * 8 * NT + g].x);
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const float2 ml = wml[w * 8 * NT + g];
-        l += (ml.x == -INFINITY) ? 0.f : ex2_approx(ml.x - M) * ml.y;
-      }
-      st_cluster_v2(cluster_map(smem_u32(&pml[part * group + g]), r), M, l);
-    }
-  }
+  const int log_dims = kLogD - (exchange ? __ffs(n_parts) - 1 : 0);  // dimensions per block
+  const int dims = 1 << log_dims;
+  if (exchange) cluster_wait();  // every block of the cluster has started and initialised its barrier
   for (int e4 = tid; e4 < group * (D / 4); e4 += kWarps * 32) {
-    const int g = e4 / (D / 4), d = (e4 % (D / 4)) * 4;
+    const int g = e4 / (D / 4), j = e4 % (D / 4), d = j * 4;
     float2 ml[kWarps];
     float M = -INFINITY;
 #pragma unroll
@@ -569,9 +581,11 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
     }
     const int h = kvh * group + g;
     if (exchange) {
-      // the block whose slice holds these four values gets them
-      const int e = g * D + d, r = e / slice;
-      st_cluster_v4(cluster_map(smem_u32(&pbuf[part * slice + (e - r * slice)]), r), o);
+      // the block that finishes these four dimensions gets them, and (from one lane each) every block the (max, sum)
+      const uint32_t bar_addr = smem_u32(arrived);
+      const int rank = d >> log_dims;
+      st_async_v4(cluster_map(smem_u32(&pbuf[(((part * group + g) << log_dims) + d) - (rank << log_dims)]), rank), o, cluster_map(bar_addr, rank));
+      if (j < n_parts) st_async_v2(cluster_map(smem_u32(&pml[part * group + g]), j), M, l, cluster_map(bar_addr, j));
     } else if (clustered) {
       const float inv = l > 0.f ? 1.f / l : 0.f;
       uint8_t* op = reinterpret_cast<uint8_t*>(a.out) +
@@ -584,21 +598,30 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
     }
   }
   if (!exchange) return;
-  // ---- merge the cluster's blocks: each finishes its slice of the output ----
-  __syncwarp();
-  cluster_arrive();
-  cluster_wait();
-  for (int t = 2 * tid; t < slice; t += 2 * kWarps * 32) {
-    const int e = part * slice + t, g = e / D, d = e % D;
+  // ---- merge the cluster's blocks: each finishes its dimensions once every block's values have arrived (a block that
+  // has sent its own and received the others' has nothing more to do with them) ----
+  if (!mbar_wait(arrived, 0, abort_flag)) {
+    report_wait(a.status, part);
+    return;
+  }
+  for (int t = 2 * tid; t < (group << log_dims); t += 2 * kWarps * 32) {
+    const int g = t >> log_dims, d = (part << log_dims) + (t & (dims - 1));
+    float2 ml[kMaxParts], x[kMaxParts];
     float M = -INFINITY, l = 0.f, o0 = 0.f, o1 = 0.f;
-    for (int p = 0; p < n_parts; ++p) M = fmaxf(M, pml[p * group + g].x);
-    for (int p = 0; p < n_parts; ++p) {
-      const float2 ml = pml[p * group + g];
-      const float sc = (ml.x == -INFINITY) ? 0.f : ex2_approx(ml.x - M);
-      const float2 x = *reinterpret_cast<const float2*>(&pbuf[p * slice + t]);
-      o0 += sc * x.x;
-      o1 += sc * x.y;
-      l += sc * ml.y;
+#pragma unroll
+    for (int p = 0; p < kMaxParts; ++p) {
+      const int q = p < n_parts ? p : 0;
+      ml[p] = pml[q * group + g];
+      x[p] = *reinterpret_cast<const float2*>(&pbuf[((q * group) << log_dims) + t]);
+      if (p >= n_parts) ml[p].x = -INFINITY;
+      M = fmaxf(M, ml[p].x);
+    }
+#pragma unroll
+    for (int p = 0; p < kMaxParts; ++p) {
+      const float sc = (ml[p].x == -INFINITY) ? 0.f : ex2_approx(ml[p].x - M);
+      o0 += sc * x[p].x;
+      o1 += sc * x[p].y;
+      l += sc * ml[p].y;
     }
     const float inv = l > 0.f ? 1.f / l : 0.f;
     uint8_t* op = reinterpret_cast<uint8_t*>(a.out) + 2 * (static_cast<size_t>(b) * a.out_stride[0] +
