@@ -26,6 +26,9 @@ HEADERS = ["attn_internal.h", "ptx.cuh"]
 # the LibTorch stable-ABI registration unit (schemas + CUDA impls that call the C ABI), host code only
 BINDING_NAME = "_C.abi3.so"
 BINDING_SOURCES = ["torch_binding/reg.cpp", "torch_binding/reg_cuda.cpp"]
+BINDING_HEADERS = ["torch_binding/attn_ops.h", "torch_binding/buffers.h"]
+# the entry points that skip the dispatcher (torch's own C++ headers, this interpreter), on top of both libraries
+DIRECT_SOURCE = "torch_binding/direct.cpp"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -66,7 +69,8 @@ def build_binding(force: bool = False, verbose: bool = False) -> str:
     import torch
     out = binding_path()
     srcs = [os.path.join(CSRC, f) for f in BINDING_SOURCES]
-    newest = max(os.path.getmtime(f) for f in srcs + [os.path.join(INCLUDE, "minfer_attn.h")])
+    newest = max(os.path.getmtime(f) for f in srcs + [os.path.join(CSRC, f) for f in BINDING_HEADERS] +
+                 [os.path.join(INCLUDE, "minfer_attn.h")])
     if not force and os.path.exists(out) and os.path.getmtime(out) >= max(newest, os.path.getmtime(lib_path())):
         return out
     tdir = os.path.dirname(torch.__file__)
@@ -89,12 +93,42 @@ def build_binding(force: bool = False, verbose: bool = False) -> str:
     return out
 
 
+def direct_path() -> str:
+    import sysconfig
+    return os.path.join(OUT_DIR, "_direct" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_direct(force: bool = False, verbose: bool = False) -> str:
+    """Compile `minfer.kernels.torch_ext._direct` against torch's C++ headers and link it to _C and the library."""
+    import sysconfig
+
+    import torch
+    out = direct_path()
+    src = os.path.join(CSRC, DIRECT_SOURCE)
+    newest = max(os.path.getmtime(f) for f in [src] + [os.path.join(CSRC, f) for f in BINDING_HEADERS] +
+                 [os.path.join(INCLUDE, "minfer_attn.h"), binding_path()])
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
+        return out
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_find_nvcc()))
+    cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", os.path.join(tdir, "include"), "-I", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include"), src, "-o", out,
+           "-L", OUT_DIR, "-l:" + BINDING_NAME, "-l:" + LIB_NAME, "-Wl,-rpath,$ORIGIN",
+           "-L", os.path.join(tdir, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+    return out
+
+
 def build(force: bool = False, verbose: bool = False, binding: bool = True) -> str:
-    """Compile if the library is missing or older than its sources (and the torch extension on top of it);
+    """Compile if the library is missing or older than its sources (and the torch extensions on top of it);
     return the library's path."""
     out = _build_library(force, verbose)
     if binding:
         build_binding(force, verbose)
+        build_direct(force, verbose)
     return out
 
 

@@ -243,13 +243,13 @@ int minfer_attn_prefill(const MinferAttnPrefillParams* p, void* stream) {
 
   static_assert(MINFER_ATTN_MAX_PEER_OUT == kMaxPeerOut, "peer output count");
   alignas(64) PeerMaps peers;
-  for (int i = 0; i < kMaxPeerOut; ++i) {
-    // unused entries repeat the local map, so that the kernel's parameter block never holds garbage
+  for (int i = 0; i < p->n_peer_out; ++i) {
     int32_t pos_unused[3];
-    void* base = i < p->n_peer_out ? p->peer_out[i] : p->out;
-    rc = make_tensor_map(&peers.m[i], base, bf16, p->head_dim, p->batch, p->n_heads, p->seq_q, p->out_stride, pos_unused, 32);
+    rc = make_tensor_map(&peers.m[i], p->peer_out[i], bf16, p->head_dim, p->batch, p->n_heads, p->seq_q, p->out_stride, pos_unused, 32);
     if (rc != MINFER_ATTN_OK) return rc;
   }
+  // unused entries repeat the local map, so that the kernel's parameter block never holds garbage
+  for (int i = p->n_peer_out; i < kMaxPeerOut; ++i) peers.m[i] = to;
   a.n_peers = p->n_peer_out;
 
   a.out = p->out;

@@ -16,6 +16,10 @@ only adds the fake implementations and the ops it does not cover.  Otherwise -
 or with MINFER_ATTN_BINDING=ctypes - the schemas are defined here with
 torch.library and every op is a Python function that fills the C-ABI structs
 through ctypes.  Both paths end in the same extern "C" entry points.
+
+With the extension, the functions below first offer a call to `_direct`, which skips the dispatcher (an eager call on
+tiny tensors costs 3 us of host time instead of 7); the ops remain what compilers, tracers, autograd, profilers and
+callers of torch.ops.minfer see, and where every error comes from.
 """
 from __future__ import annotations
 
@@ -83,6 +87,15 @@ if _binding_choice != "ctypes":
             raise
         _C = None
 BINDING = "stable" if _C is not None else "ctypes"
+# entry points that skip the dispatcher (csrc/torch_binding/direct.cpp): each returns whether it served the call, which
+# it does for plain CUDA tensors on the current device with nothing on the thread that wants to see the op
+_direct = None
+if _C is not None and _binding_choice == "auto":
+    try:
+        from . import _direct
+    except ImportError:
+        _direct = None
+_is_compiling = torch.compiler.is_compiling  # a tracer has to meet the op itself
 # ops whose CUDA implementation lives in the extension
 _IN_EXTENSION = tuple(_DEFS) if _C is not None else ()
 
@@ -404,11 +417,15 @@ def flash_attn(
     q/out: [B, n_heads, L, D], k/v: [B, n_kv_heads, L, D]; the three leading ints are unused
     by attention, as in the reference.
     """
+    if _direct is not None and not _is_compiling() and _direct.flash_attn(qtype_int, qblock_size, qtype_size, q, k, v, mask, out):
+        return None
     return torch.ops.minfer.flash_attn.default(qtype_int, qblock_size, qtype_size, q, k, v, mask, out)
 
 
 def flash_attn_causal(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor):
     """causal attention (key j visible to query i iff j <= i + Lk - Lq) without a materialised mask."""
+    if _direct is not None and not _is_compiling() and _direct.flash_attn_causal(q, k, v, out):
+        return None
     return torch.ops.minfer.flash_attn_causal.default(q, k, v, out)
 
 
@@ -418,6 +435,8 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     one-token decode over a padded KV cache: q/out [B, n_heads, 1, D], caches
     [B, n_kv_heads, max_len, D], lens int32 [B]; sequence b attends keys [0, lens[b]).
     """
+    if _direct is not None and not _is_compiling() and _direct.flash_attn_decode(q, k_cache, v_cache, lens, out):
+        return None
     return torch.ops.minfer.flash_attn_decode.default(q, k_cache, v_cache, lens, out)
 
 
@@ -428,6 +447,8 @@ def flash_attn_decode_paged(q: torch.Tensor, k_pages: torch.Tensor, v_pages: tor
     of 16), block_table int32 [B, max_pages]; key j of sequence b is row j % page_size of page
     block_table[b, j // page_size].  Only the entries below ceil(lens[b] / page_size) are read.
     """
+    if _direct is not None and not _is_compiling() and _direct.flash_attn_decode_paged(q, k_pages, v_pages, block_table, lens, out):
+        return None
     return torch.ops.minfer.flash_attn_decode_paged.default(q, k_pages, v_pages, block_table, lens, out)
 
 
@@ -435,6 +456,8 @@ def il_rope(rotary_dim: int, start_pos: int, freq_base: float, x: torch.Tensor):
     """
     Applies il_rope in-place (per-head): interleaved pairs of x [B, L, n_heads, head_dim]
     """
+    if _direct is not None and not _is_compiling() and _direct.il_rope(rotary_dim, start_pos, freq_base, x):
+        return None
     return torch.ops.minfer.il_rope.default(rotary_dim, start_pos, freq_base, x)
 
 
@@ -442,6 +465,8 @@ def neox_rope(rotary_dim: int, start_pos: int, freq_base: float, x: torch.Tensor
     """
     Applies neox_rope in-place (per-head): halves of x [B, L, n_heads, head_dim]
     """
+    if _direct is not None and not _is_compiling() and _direct.neox_rope(rotary_dim, start_pos, freq_base, x):
+        return None
     return torch.ops.minfer.neox_rope.default(rotary_dim, start_pos, freq_base, x)
 
 
@@ -452,6 +477,8 @@ def rope_kv_append(rotary_dim: int, freq_base: float, style: int, q: torch.Tenso
     [B, L, Hkv, D] into the caches [B, Hkv, Lmax, D] at rows start[b] + l (start: int32 [B]).
     style 0 = interleaved (il_rope), 1 = neox.
     """
+    if _direct is not None and not _is_compiling() and _direct.rope_kv_append(rotary_dim, freq_base, style, q, k, v, k_cache, v_cache, start):
+        return None
     return torch.ops.minfer.rope_kv_append.default(rotary_dim, freq_base, style, q, k, v, k_cache, v_cache, start)
 
 
@@ -461,6 +488,8 @@ def flash_attn_decode_q8(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
     flash_attn_decode over a GGML Q8_0 KV cache: caches are uint8 [B, n_kv_heads, max_len, D/32*34]
     (32 int8 + one fp16 scale per block); equals flash_attn_decode on the dequantised cache.
     """
+    if _direct is not None and not _is_compiling() and _direct.flash_attn_decode_q8(q, k_cache, v_cache, lens, out):
+        return None
     return torch.ops.minfer.flash_attn_decode_q8.default(q, k_cache, v_cache, lens, out)
 
 
@@ -469,6 +498,9 @@ def rope_kv_append_paged(rotary_dim: int, freq_base: float, style: int, q: torch
                          start: torch.Tensor):
     """rope_kv_append into a paged cache: pools [n_pages, Hkv, page_size, D], block_table int32 [B, max_pages];
     position p of sequence b goes to row p % page_size of page block_table[b, p // page_size]."""
+    if _direct is not None and not _is_compiling() and _direct.rope_kv_append_paged(
+            rotary_dim, freq_base, style, q, k, v, k_pages, v_pages, block_table, start):
+        return None
     return torch.ops.minfer.rope_kv_append_paged.default(rotary_dim, freq_base, style, q, k, v, k_pages, v_pages,
                                                          block_table, start)
 
@@ -476,6 +508,8 @@ def rope_kv_append_paged(rotary_dim: int, freq_base: float, style: int, q: torch
 def rope_kv_append_q8(rotary_dim: int, freq_base: float, style: int, q: torch.Tensor, k: torch.Tensor,
                       v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, start: torch.Tensor):
     """rope_kv_append into GGML Q8_0 caches: the rows the 16-bit cache would get, quantised block by block."""
+    if _direct is not None and not _is_compiling() and _direct.rope_kv_append_q8(rotary_dim, freq_base, style, q, k, v, k_cache, v_cache, start):
+        return None
     return torch.ops.minfer.rope_kv_append_q8.default(rotary_dim, freq_base, style, q, k, v, k_cache, v_cache, start)
 
 

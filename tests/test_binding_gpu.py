@@ -88,3 +88,72 @@ def test_extension_argument_errors_are_runtime_errors(kerns):
         kerns.flash_attn_causal(q, k, k, torch.zeros(1, 4, 128, 64, dtype=torch.float16, device="cuda"))
     with pytest.raises(RuntimeError):
         kerns.flash_attn_decode(q[:, :, :1], k, k, torch.zeros(1, dtype=torch.int64, device="cuda"), torch.zeros_like(q[:, :, :1]))
+
+
+def _op_calls():
+    """Arguments of one small call per op (fresh tensors, the same values every time) and which of them it writes."""
+    g = torch.Generator().manual_seed(21)
+    r = lambda *s: torch.randn(*s, generator=g).half().cuda()  # noqa: E731
+    B, H, Hkv, L, D, page = 2, 4, 2, 48, 64, 16
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    q, k, v, qd = r(B, H, L, D), r(B, Hkv, L, D), r(B, Hkv, L, D), r(B, H, 1, D)
+    q8 = [O.q8_0_quantize(torch.randn(B, Hkv, L, D, generator=g).half()).cuda() for _ in range(2)]
+    pools, table, lens = [r(6, Hkv, page, D) for _ in range(2)], i32([[5, 0, 2], [1, 4, 3]]), i32([48, 17])
+    mask = (torch.rand(B, 1, L, L, generator=g) < 0.5).cuda()
+    tok, kt, vt = r(B, 3, H, D), r(B, 3, Hkv, D), r(B, 3, Hkv, D)
+    return {
+        "flash_attn": ([1, 1, 2, q, k, v, mask, torch.zeros_like(q)], [7]),
+        "flash_attn_causal": ([q, k, v, torch.zeros_like(q)], [3]),
+        "flash_attn_decode": ([qd, k, v, lens, torch.zeros_like(qd)], [4]),
+        "flash_attn_decode_q8": ([qd, *q8, lens, torch.zeros_like(qd)], [4]),
+        "flash_attn_decode_paged": ([qd, *pools, table, lens, torch.zeros_like(qd)], [5]),
+        "il_rope": ([D, 7, 10000.0, tok], [3]),
+        "neox_rope": ([D, 7, 10000.0, tok], [3]),
+        "rope_kv_append": ([D, 10000.0, 1, tok, kt, vt, k, v, i32([0, 40])], [3, 6, 7]),
+        "rope_kv_append_q8": ([D, 10000.0, 0, tok, kt, vt, *q8, i32([0, 40])], [3, 6, 7]),
+        "rope_kv_append_paged": ([D, 10000.0, 0, tok, kt, vt, *pools, table, i32([0, 40])], [3, 6, 7]),
+    }
+
+
+@pytest.mark.parametrize("name", ["flash_attn", "flash_attn_causal", "flash_attn_decode", "flash_attn_decode_q8", "flash_attn_decode_paged",
+                                  "il_rope", "neox_rope", "rope_kv_append", "rope_kv_append_q8", "rope_kv_append_paged"])
+def test_direct_entry_point_gives_the_bits_of_the_dispatched_op(name):
+    from minfer.kernels.torch_ext import ops
+    assert ops._direct is not None, "the direct entry points were not built"
+    a, written = _op_calls()[name]
+    b, _ = _op_calls()[name]
+    assert getattr(ops._direct, name)(*a) is True
+    getattr(torch.ops.minfer, name).default(*b)
+    for i in written:
+        assert torch.equal(a[i], b[i]), f"{name}: argument {i}"
+
+
+def test_direct_entry_points_leave_everything_unusual_to_the_dispatcher(kerns):
+    """Wrong arguments, autograd, modes and tracers: the direct call declines (and writes nothing), the façade behaves as the op."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from minfer.kernels.torch_ext import ops
+    f = ops._direct.flash_attn_decode
+    q, k, v, lens, out = _op_calls()["flash_attn_decode"][0]
+    out.fill_(7.0)
+    assert f(q, k, v, lens.long(), out) is False and f(q, k, v, lens, out[..., :32]) is False and f(q, k, v, lens) is False
+    assert f(q.cpu(), k, v, lens, out) is False and f(q.float(), k, v, lens, out) is False
+    assert f(torch.nn.Parameter(q), k, v, lens, out) is False
+    assert f(q.clone().requires_grad_(), k, v, lens, out) is False
+
+    class Sees(TorchDispatchMode):
+        seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Sees() as mode:
+        assert f(q, k, v, lens, out) is False
+        assert (out == 7.0).all()
+        kerns.flash_attn_decode(q, k, v, lens, out)
+        assert "minfer.flash_attn_decode.default" in mode.seen
+    with torch.inference_mode():
+        assert f(q, k, v, lens, torch.zeros_like(q)) is True
+    out2 = torch.zeros_like(out)
+    torch.compile(lambda o: kerns.flash_attn_decode(q, k, v, lens, o), fullgraph=True, backend="eager")(out2)
+    assert torch.equal(out, out2)
