@@ -14,10 +14,12 @@
 // m16n8k16 tile and query heads as its 8 columns, because a GQA group is rarely more than 8.  With the heads as rows
 // half of every MMA, of the accumulators and of the exponentials belonged to rows that do not exist; transposed, a
 // 16-key tile takes half the MMAs and 4 exponentials per lane (groups of 9-16 take two column tiles).  P^T comes
-// from S^T by two 8x8 transposes (movmatrix) per tile.  The reference maximum moves only when a score exceeds it by
-// 2^8, so ordinary tiles need no reduction over lanes.  (Counted from the source, a Q8_0 tile takes some 430 warp
-// instructions, 780 were measured before;
-// the batch-64 Q8_0 call 147 -> 107 us, 5.2 of 6.5 TB/s.)
+// from S^T by two 8x8 transposes (movmatrix) per tile.  A tile in which no score exceeds
+// its row's maximum so far needs no reduction over lanes.  (Counted from the source, a Q8_0 tile takes some 430 warp
+// instructions, 780 were measured before; the batch-64 Q8_0 call 147 -> 110 us, 5.1 of 6.5 TB/s.)  The maximum is exact:
+// letting it lag by up to 2^8, as the prefill kernel does, saves the batch-64 calls 1 % (16-bit) and 3 % (Q8_0), but the
+// largest weights are then no longer just below 1, where 16 bits round them best: error against 64 bits 2.9e-4 instead
+// of 2.6e-4 of the output at float16.
 //
 // The blocks of one (sequence, kv head) form a cluster: they share the sequence's actual tiles evenly - a padded
 // cache has no empty blocks - and each pushes its partial output into the shared memory of the block that finishes
@@ -63,7 +65,6 @@ constexpr int kMaxRanked = 256;  // sequences a block ranks by length
 #define MINFER_ATTN_Q8_STAGES 4
 #endif
 constexpr int kTileKeys = 16;
-constexpr float kMoveThreshold = 8.0f;  // log2 units
 
 // Shared memory of a decode block: the warps' rings (reused for their partial outputs), then what the merges need.
 template <int D, bool Q8, int NT>
@@ -411,8 +412,8 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[n][e] += s2[n][e];
 
-    // ---- online softmax over the keys: x = s * scale - reference; the reference moves only when a score exceeds it
-    // by 2^8 (weights stay below 256, sums in fp32), so that ordinary tiles need no reduction over the lanes ----
+    // ---- online softmax over the keys: x = s * scale - maximum so far; a tile in which no score exceeds it needs no
+    // reduction over the lanes ----
     const bool partial = key0 + kTileKeys > c1;
     const bool dead0 = partial && key0 + g0 >= c1, dead1 = partial && key0 + g0 + 8 >= c1;
     float x[NT][4];
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
         x[n][e] = fmaf(s[n][e], sl2, -m_ref[n][e & 1]);  // +inf before the first tile
         if (e < 2 ? dead0 : dead1) x[n][e] = -INFINITY;
       }
-      move |= fmaxf(fmaxf(x[n][0], x[n][1]), fmaxf(x[n][2], x[n][3])) > kMoveThreshold;
+      move |= fmaxf(fmaxf(x[n][0], x[n][1]), fmaxf(x[n][2], x[n][3])) > 0.f;
     }
     if (__any_sync(0xFFFFFFFFu, move)) {
 #pragma unroll
@@ -587,10 +588,12 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
       st_async_v4(cluster_map(smem_u32(&pbuf[(((part * group + g) << log_dims) + d) - (rank << log_dims)]), rank), o, cluster_map(bar_addr, rank));
       if (j < n_parts) st_async_v2(cluster_map(smem_u32(&pml[part * group + g]), j), M, l, cluster_map(bar_addr, j));
     } else if (clustered) {
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float inv = 1.f / l;
+      if (!(l > 0.f)) o = make_float4(0.f, 0.f, 0.f, 0.f);  // no key, or a sum that is NaN
+      else o = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
       uint8_t* op = reinterpret_cast<uint8_t*>(a.out) +
                     2 * (static_cast<size_t>(b) * a.out_stride[0] + static_cast<size_t>(h) * a.out_stride[1] + d);
-      *reinterpret_cast<uint2*>(op) = make_uint2(pack2<BF16>(o.x * inv, o.y * inv), pack2<BF16>(o.z * inv, o.w * inv));
+      *reinterpret_cast<uint2*>(op) = make_uint2(pack2<BF16>(o.x, o.y), pack2<BF16>(o.z, o.w));
     } else {
       const size_t pidx = (static_cast<size_t>(b) * a.n_heads + h) * n_parts + part;
       *reinterpret_cast<float4*>(a.part_o + pidx * D + d) = o;
@@ -613,7 +616,10 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
       const int q = p < n_parts ? p : 0;
       ml[p] = pml[q * group + g];
       x[p] = *reinterpret_cast<const float2*>(&pbuf[((q * group) << log_dims) + t]);
-      if (p >= n_parts) ml[p].x = -INFINITY;
+      if (p >= n_parts) {  // counts for nothing, whatever part 0 holds
+        ml[p] = make_float2(-INFINITY, 0.f);
+        x[p] = make_float2(0.f, 0.f);
+      }
       M = fmaxf(M, ml[p].x);
     }
 #pragma unroll
@@ -623,10 +629,12 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
       o1 += sc * x[p].y;
       l += sc * ml[p].y;
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
+    const float inv = 1.f / l;
+    o0 = l > 0.f ? o0 * inv : 0.f;
+    o1 = l > 0.f ? o1 * inv : 0.f;
     uint8_t* op = reinterpret_cast<uint8_t*>(a.out) + 2 * (static_cast<size_t>(b) * a.out_stride[0] +
                                                            static_cast<size_t>(kvh * group + g) * a.out_stride[1] + d);
-    *reinterpret_cast<uint32_t*>(op) = pack2<BF16>(o0 * inv, o1 * inv);
+    *reinterpret_cast<uint32_t*>(op) = pack2<BF16>(o0, o1);
   }
 }
 

@@ -205,3 +205,25 @@ def test_block_clusters_and_order_by_length(kerns, B, Hkv, group, D, Lmax, dtype
     else:
         check_close(got[live], want[live], f"B={B} D={D}")
     assert torch.equal(got, run_decode(kerns, q, kc, vc, lens))
+
+
+@pytest.mark.parametrize("D,H,Hkv,Lmax", [(128, 8, 2, 700), (64, 4, 4, 700), (64, 12, 1, 100), (128, 2, 1, 20)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_infinite_values_and_nan_scores(kerns, D, H, Hkv, Lmax, dtype):
+    """A visible infinite value makes its dimension infinite and nothing else NaN, whatever the number of blocks that share
+    the sequence; a row whose sum of weights is NaN (a NaN key or query) is zeros, as the merging kernel has it."""
+    B = 3
+    g = torch.Generator().manual_seed(D + H)
+    q = torch.randn(B, H, 1, D, generator=g).to(dtype)
+    kc = torch.randn(B, Hkv, Lmax, D, generator=g).to(dtype)
+    vc = torch.randn(B, Hkv, Lmax, D, generator=g).to(dtype)
+    lens = torch.tensor([Lmax - 1, 11, Lmax // 2], dtype=torch.int32)
+    want = O.attention_f64(q, kc, vc, lens=lens)
+    vc[:, :, 7, 3] = float("inf")
+    kc[1, :, 10] = float("nan")
+    q[2] = float("nan")
+    got = run_decode(kerns, q, kc, vc, lens).float().cpu()
+    assert (got[0, ..., 3] == float("inf")).all()
+    keep = [d for d in range(D) if d != 3]
+    check_close(got[:1][..., keep], want[:1][..., keep], "finite dimensions", bf16=dtype == torch.bfloat16)
+    assert torch.count_nonzero(got[1:]) == 0
