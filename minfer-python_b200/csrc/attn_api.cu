@@ -268,7 +268,7 @@ int minfer_attn_prefill(const MinferAttnPrefillParams* p, void* stream) {
       uint32_t* bits = nullptr;
       if (p->workspace_bytes >= minfer_attn_prefill_workspace_bytes_bits(p->batch, p->seq_q, p->seq_k))
         bits = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(p->workspace) + ((need + 15) & ~static_cast<size_t>(15)));
-      cudaError_t ce = launch_mask_classify(a.mask, cls, bits, p->batch, p->seq_q, p->seq_k, static_cast<cudaStream_t>(stream));
+      cudaError_t ce = launch_mask_classify(a.mask, cls, bits, a.counter, p->batch, p->seq_q, p->seq_k, static_cast<cudaStream_t>(stream));
       if (ce != cudaSuccess) return cuda_result(ce);
       a.cls = cls;
       a.bits = bits;

@@ -54,6 +54,7 @@ struct PrefillArgs {
   int32_t n_peers;        // output replicas on other GPUs: every output tile is also stored through PeerMaps::m[0 .. n_peers)
   int32_t items_x, items_y;  // persistent kernel: work-item grid (query tile [pairs], head [pairs]); set by its launcher
   int32_t order_by_kv_set;   // persistent kernel, dynamic claiming: item order (see its launcher)
+  int programmatic;       // launched beside the kernel in front of it, and lets the one behind do the same
   float scale_log2;       // softmax scale * log2(e)
   // position (1..3) of the batch / head / row coordinate inside each tensor
   // map; coordinate 0 is always head_dim
@@ -74,9 +75,9 @@ cudaError_t launch_prefill_persist(const CUtensorMap& tq, const CUtensorMap& tk,
 
 // Classifies every 128 x 128 tile of a dense [batch, 1, seq_q, seq_k] byte mask: 0 = no byte set,
 // 1 = every in-range byte set, 2 = mixed.  cls is [batch, ceil(seq_q/128), ceil(seq_k/128)]; bits (or null): per tile
-// of cls, 128 rows of 128 bits, written for mixed tiles only.
-cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, uint32_t* bits, int batch, int seq_q, int seq_k,
-                                 cudaStream_t stream);
+// of cls, 128 rows of 128 bits, written for mixed tiles only.  counter: set to zero.
+cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, uint32_t* bits, int* counter, int batch, int seq_q,
+                                 int seq_k, cudaStream_t stream);
 
 // Kernel-side view of a RoPE + KV-append call.  Strides in elements.
 struct RopeArgs {

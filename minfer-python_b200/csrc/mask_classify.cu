@@ -16,11 +16,12 @@ namespace {
 
 constexpr int kTile = 128;
 
-// 16 columns of one mask row as words.
-__device__ __forceinline__ void row_words16(const uint8_t* __restrict__ p, uint32_t (&w)[4]) {
+// 16 columns of one mask row as words.  (Ordinary loads: the kernel starts beside the one that may write the mask, and
+// the read-only path is for memory that nobody writes during the kernel's life.)
+__device__ __forceinline__ void row_words16(const uint8_t* p, uint32_t (&w)[4]) {
   const uint32_t mis = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)) & 15u;
   if (mis == 0) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
     w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
   } else {
     // rows of a mask whose length is no multiple of 16 start anywhere: aligned words, shifted into place (every
@@ -29,8 +30,8 @@ __device__ __forceinline__ void row_words16(const uint8_t* __restrict__ p, uint3
     const uint32_t sh = (mis & 3u) * 8u;
     uint32_t a[5];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = __ldg(q + i);
-    a[4] = sh ? __ldg(q + 4) : 0u;
+    for (int i = 0; i < 4; ++i) a[i] = q[i];
+    a[4] = sh ? q[4] : 0u;
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(a[i], a[i + 1], sh);
   }
@@ -42,8 +43,12 @@ __device__ __forceinline__ void row_words16(const uint8_t* __restrict__ p, uint3
 // instruction-bound.  Mixed tiles then leave their bits behind (128 rows of 16 bytes), so that the attention
 // kernel, which needs a mixed tile once per head pair, reads 16 bytes per row instead of 128 and no row of it is
 // misaligned.
-__global__ void __launch_bounds__(256, 6) mask_classify_kernel(const uint8_t* __restrict__ mask, uint8_t* __restrict__ cls,
-                                                            uint32_t* __restrict__ bits, int seq_q, int seq_k) {
+__global__ void __launch_bounds__(256, 6) mask_classify_kernel(const uint8_t* mask, uint8_t* cls, uint32_t* bits,
+                                                               int* counter, int seq_q, int seq_k) {
+  grid_launch_dependents();  // the attention kernel sets up beside the last blocks of this pass
+  grid_dependency_wait();
+  // its work-item counter starts at zero
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) *counter = 0;
   const int kt = blockIdx.x, qt = blockIdx.y, b = blockIdx.z;
   const int part = threadIdx.x & 7;
   const int r0 = static_cast<int>(threadIdx.x) >> 3;
@@ -106,11 +111,12 @@ __global__ void __launch_bounds__(256, 6) mask_classify_kernel(const uint8_t* __
 
 }  // namespace
 
-cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, uint32_t* bits, int batch, int seq_q, int seq_k,
-                                 cudaStream_t stream) {
-  dim3 grid((seq_k + kTile - 1) / kTile, (seq_q + kTile - 1) / kTile, batch);
-  mask_classify_kernel<<<grid, 256, 0, stream>>>(mask, cls, bits, seq_q, seq_k);
-  return cudaGetLastError();
+cudaError_t launch_mask_classify(const uint8_t* mask, uint8_t* cls, uint32_t* bits, int* counter, int batch, int seq_q,
+                                 int seq_k, cudaStream_t stream) {
+  LaunchAttrs at(stream);
+  at.cfg.gridDim = dim3((seq_k + kTile - 1) / kTile, (seq_q + kTile - 1) / kTile, batch);
+  at.cfg.blockDim = dim3(256);
+  return cudaLaunchKernelEx(&at.cfg, mask_classify_kernel, mask, cls, bits, counter, seq_q, seq_k);
 }
 
 }  // namespace minfer_attn

@@ -522,3 +522,35 @@ def test_mask_tile_bits_at_unaligned_rows(kerns, L, offset):
         outs.append(out)
     assert torch.equal(outs[0], outs[1])
     check_close(outs[0], O.attention_f64(q.cpu(), k.cpu(), v.cpu(), mask=m != 0), f"bits L={L} offset={offset}")
+
+
+@pytest.mark.parametrize("L,H", [(40, 2), (300, 4), (700, 32)])
+def test_calls_of_one_stream_in_a_row(kerns, L, H):
+    """Kernels of neighbouring calls are resident together: each call's mask, queries and work-item counter (one workspace
+    for all; items below and above the number of SMs) must be its own.  Against the same calls, each waited for."""
+    B, Hkv, D, n = 2, 2, 64, 6
+    sets = [tuple(x.cuda() for x in seeded_qkv(50 + i, B, H, Hkv, L, L, D, torch.float16)) for i in range(n)]
+    g = torch.Generator(device="cuda").manual_seed(L)
+    masks = [torch.rand(B, 1, L, L, generator=g, device="cuda") < 0.1 + 0.15 * i for i in range(n)]
+
+    def run(wait):
+        q, k, v = (x.clone() for x in sets[0])
+        mask = torch.empty_like(masks[0])
+        outs = []
+        for (qi, ki, vi), mi in zip(sets, masks):
+            q.copy_(qi), k.copy_(ki), v.copy_(vi), mask.copy_(mi)
+            pair = [torch.zeros_like(q) for _ in range(3)]
+            kerns.flash_attn(*F16, q, k, v, mask, pair[0])
+            kerns.flash_attn_causal(pair[0], k, v, pair[1])     # reads what the call in front writes
+            kerns.flash_attn(*F16, pair[1], k, v, mask, pair[2])
+            if wait:
+                torch.cuda.synchronize()
+            outs += pair
+        torch.cuda.synchronize()
+        return outs
+
+    want = run(True)
+    for _ in range(3):
+        for a, b in zip(run(False), want):
+            assert torch.equal(a, b)
+    check_close(want[0], O.attention_f64(*(x.cpu() for x in sets[0]), mask=masks[0].cpu()), f"L={L} H={H}")
