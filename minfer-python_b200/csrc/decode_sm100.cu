@@ -259,7 +259,9 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
     const size_t head_off = kUnit * static_cast<size_t>(kvh) * a.kv_stride[1];
     if constexpr (Paged) {
       const int slot = key0 / a.page_size;
-      int page = __ldg(a.block_table + static_cast<size_t>(b) * a.table_stride + slot);
+      // (an ordinary load: the read-only path is for memory that nobody writes while this kernel is resident, and it is
+      // resident before the kernel in front, which may write the table, has ended)
+      int page = a.block_table[static_cast<size_t>(b) * a.table_stride + slot];
       if (static_cast<unsigned>(page) >= static_cast<unsigned>(a.n_pages)) {
         // never follow an entry that points outside the pools: report it and read page 0 instead
         if (lane == 0) report_bad_page(a.status, b, slot, page);
