@@ -142,10 +142,11 @@ __device__ __forceinline__ uint32_t ld_q8_word(const uint8_t* p, bool aligned4) 
 // The sequence that is i-th when the batch is ordered by descending length (ties by index); every block finds its own.
 // Blocks start in grid order, so the long sequences start first and the last wave holds the short ones.  Four lengths
 // per shared-memory read, the reads of one sequence dealt out over the lanes a small batch leaves free.  Returns the
-// sequence and its length.
-__device__ __forceinline__ int2 sequence_by_length(const int32_t* lens, int batch, int i, int* scratch, int tid) {
+// sequence and its length.  The lengths are clamped to [0, max_len] before they are ranked: only then is every one of them
+// above the padding (-1), `mine + 1` exact, and every rank taken once.
+__device__ __forceinline__ int2 sequence_by_length(const int32_t* lens, int batch, int max_len, int i, int* scratch, int tid) {
   const int n4 = (batch + 3) / 4;
-  for (int t = tid; t < 4 * n4; t += kWarps * 32) scratch[t] = t < batch ? lens[t] : -1;
+  for (int t = tid; t < 4 * n4; t += kWarps * 32) scratch[t] = t < batch ? max(0, min(lens[t], max_len)) : -1;
   int lanes = 1;  // per sequence
   while (lanes < 16 && 2 * lanes * batch <= kWarps * 32) lanes *= 2;
   __syncthreads();
@@ -227,13 +228,12 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
   // ---- which sequence: in order, or the i-th longest (a.by_length: few enough sequences to rank them here) ----
   int b = blockIdx.z, len;
   if (a.by_length) {
-    const int2 x = sequence_by_length(a.lens, a.batch, b, reinterpret_cast<int*>(smem), tid);
+    const int2 x = sequence_by_length(a.lens, a.batch, a.max_len, b, reinterpret_cast<int*>(smem), tid);
     b = x.x;
     len = x.y;
   } else {
-    len = a.lens[b];
+    len = max(0, min(a.lens[b], a.max_len));
   }
-  len = max(0, min(len, a.max_len));
   // ---- the keys of this block: an even share of the sequence's tiles, or the part-th chunk ----
   int c0, c1;
   if (clustered) {

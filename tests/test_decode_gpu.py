@@ -227,3 +227,29 @@ def test_infinite_values_and_nan_scores(kerns, D, H, Hkv, Lmax, dtype):
     keep = [d for d in range(D) if d != 3]
     check_close(got[:1][..., keep], want[:1][..., keep], "finite dimensions", bf16=dtype == torch.bfloat16)
     assert torch.count_nonzero(got[1:]) == 0
+
+
+@pytest.mark.parametrize("B,Hkv,Lmax", [(6, 8, 6912), (13, 8, 3264), (255, 1, 1300), (256, 1, 1300)])
+def test_lengths_outside_the_cache_are_clamped_in_order_by_length(kerns, B, Hkv, Lmax):
+    """Calls that take the longest sequences first, batches that are and are not multiples of four: a negative length is an
+    empty sequence (zeros), one beyond the cache is max_len, and no sequence is lost - the bits of the same call with clamped lengths."""
+    D, dtype = 128, torch.float16
+    g = torch.Generator(device="cuda").manual_seed(B)
+    q = torch.randn(B, Hkv, 1, D, generator=g, device="cuda", dtype=dtype)
+    kc = torch.randn(B, Hkv, Lmax, D, generator=g, device="cuda", dtype=dtype)
+    vc = torch.randn(B, Hkv, Lmax, D, generator=g, device="cuda", dtype=dtype)
+    lens = torch.randint(1, Lmax, (B,), generator=g, device="cuda", dtype=torch.int32)
+    for odd in ([-5, 2 ** 31 - 1], [-2, Lmax + 3, -2 ** 31], [2 ** 31 - 1, -1, -2, -5]):
+        bad = lens.clone()
+        bad[torch.randperm(B, generator=g, device="cuda")[:len(odd)]] = torch.tensor(odd, device="cuda", dtype=torch.int32)
+        outs = []
+        for n in (bad, bad.clamp(0, Lmax)):
+            out = torch.full((B, Hkv, 1, D), float("nan"), dtype=dtype, device="cuda")
+            kerns.flash_attn_decode(q, kc, vc, n, out)
+            outs.append(out)
+        assert torch.equal(outs[0], outs[1])
+        assert torch.count_nonzero(outs[0][bad <= 0]) == 0 and torch.isfinite(outs[0]).all()
+        full = bad > Lmax
+        if full.any():
+            want = O.attention_f64(q[full].cpu(), kc[full].cpu(), vc[full].cpu(), lens=torch.full((int(full.sum()),), Lmax, dtype=torch.int32))
+            check_close(outs[0][full], want, f"B={B} beyond the cache")
