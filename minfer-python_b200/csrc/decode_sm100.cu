@@ -90,12 +90,18 @@ __device__ __noinline__ void report_bad_page(int32_t* status, int b, int slot, i
   }
 }
 
-__device__ __noinline__ void report_wait(int32_t* status, int part) {
+// A block whose wait for the cluster's partial outputs ran out.  It reports that, and stays until nothing can be stored into
+// its shared memory any more: the barrier waits for the threads of the cluster that have not ended, so it passes when
+// every other block has sent and ended, or has given up (after sending) as well; what is then on its way completes the mbarrier.
+__device__ __noinline__ void give_up(uint64_t* arrived, int32_t* status, int part) {
   if (status != nullptr && atomicCAS(status, 0, kStatusWaitTimeout) == 0) {
     status[1] = part;
     status[2] = static_cast<int32_t>(blockIdx.z);
     status[3] = 50;
   }
+  cluster_sync_unaligned();
+  volatile int own_flag = 0;
+  mbar_wait<true>(arrived, 0, &own_flag);
 }
 
 template <int D>
@@ -605,8 +611,9 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
   if (!exchange) return;
   // ---- merge the cluster's blocks: each finishes its dimensions once every block's values have arrived (a block that
   // has sent its own and received the others' has nothing more to do with them) ----
-  if (!mbar_wait(arrived, 0, abort_flag)) {
-    report_wait(a.status, part);
+  // (their stores are released at the scope of the cluster: the wait acquires there)
+  if (!mbar_wait<true>(arrived, 0, abort_flag)) {
+    give_up(arrived, a.status, part);
     return;
   }
   for (int t = 2 * tid; t < (group << log_dims); t += 2 * kWarps * 32) {
