@@ -16,10 +16,16 @@
 // 16-key tile takes half the MMAs and 4 exponentials per lane (groups of 9-16 take two column tiles).  P^T comes
 // from S^T by two 8x8 transposes (movmatrix) per tile.  A tile in which no score exceeds
 // its row's maximum so far needs no reduction over lanes.  (Counted from the source, a Q8_0 tile takes some 430 warp
-// instructions, 780 were measured before; the batch-64 Q8_0 call 147 -> 110 us, 5.1 of 6.5 TB/s.)  The maximum is exact:
-// letting it lag by up to 2^8, as the prefill kernel does, saves the batch-64 calls 1 % (16-bit) and 3 % (Q8_0), but the
-// largest weights are then no longer just below 1, where 16 bits round them best: error against 64 bits 2.9e-4 instead
-// of 2.6e-4 of the output at float16.
+// instructions, 780 were measured before.)
+//
+// Precision: the weights are rounded to 16 bits relative to the reference maximum, so a weight of exactly 1 - the largest
+// key's so far - costs nothing, and that is worth more the fewer keys share a maximum.  Therefore the maximum is exact
+// within a segment (letting it lag by up to 2^8, as the prefill kernel does, gives 2.9e-4 of the output at float16 against
+// 64 bits), and every chunk / 64 tiles - as many as a warp has of a chunk in the form with chunks - the reference is
+// lowered by 2^4, so that the next segment's largest keys set it again.  64 sequences of 512-8192 (float16 / bfloat16): 2.57e-4 / 2.06e-3;
+// one maximum for all keys of a warp 2.65e-4 / 2.12e-3; chunks of 512 keys 2.59e-4 / 2.07e-3.  What it costs (us, with / without): 16-bit 165.6 /
+// 165.2, Q8_0 116 / 109, one sequence of 16384, 8 kv heads 15.5 / 15.1.  (A second product with the rounding errors of
+// the weights gives 2.07e-4, but an infinite value times an error of 0 is NaN.)
 //
 // The blocks of one (sequence, kv head) form a cluster: they share the sequence's actual tiles evenly - a padded
 // cache has no empty blocks - and each pushes its partial output into the shared memory of the block that finishes
@@ -362,6 +368,7 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
     l_run[n][0] = l_run[n][1] = 0.f;
   }
   const float sl2 = a.scale_log2;
+  const int seg_mask = clustered ? a.chunk / 64 - 1 : -1;  // tiles per segment (a power of two) - 1; a chunk is one segment
 
   // ldmatrix lane roles
   const int lm_mi = lane >> 3;
@@ -371,6 +378,28 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
     cp_async_wait<kSt - 2>();
     __syncwarp();
     issue_tile(i + kSt - 1);
+
+    // ---- a new segment: the reference maximum is lowered (O and the sums scaled by the same power of two, exactly), so that
+    // this segment's largest scores move it; not while a sum is large, so that a long run of falling scores cannot overflow ----
+    if ((i & seg_mask) == 0 && i > 0) {
+      bool room = true;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) room = room && fmaxf(l_run[n][0], l_run[n][1]) < 512.f;
+      if (__all_sync(0xFFFFFFFFu, room)) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            m_ref[n][h] -= 4.f;
+            l_run[n][h] *= 16.f;
+          }
+#pragma unroll
+          for (int m = 0; m < D / 16; ++m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) oacc[n][m][e] *= 16.f;
+        }
+      }
+    }
 
     const int key0 = c0 + (warp + i * kWarps) * kTileKeys;
     // ---- S^T[16 keys x 8 heads] = K Q^T ----

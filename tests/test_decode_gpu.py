@@ -253,3 +253,59 @@ def test_lengths_outside_the_cache_are_clamped_in_order_by_length(kerns, B, Hkv,
         if full.any():
             want = O.attention_f64(q[full].cpu(), kc[full].cpu(), vc[full].cpu(), lens=torch.full((int(full.sum()),), Lmax, dtype=torch.int32))
             check_close(outs[0][full], want, f"B={B} beyond the cache")
+
+
+def test_weights_keep_the_precision_of_512_key_chunks(kerns):
+    """Rounding the weights to 16 bits costs least where few keys share a reference maximum: a large call's error against 64
+    bits is no more than that of chunks of 512 keys dealt out to four warps in 16-key tiles, each with a running maximum of
+    its own.  (The two cut the keys differently; over 2048 rows that moves the error by about 0.5 %.)"""
+    B, Hkv, group, D, Lmax = 64, 8, 4, 128, 8192
+    g = torch.Generator(device="cuda").manual_seed(1)
+    lens = torch.tensor([512 + (Lmax - 512) * i // (B - 1) for i in range(B)], dtype=torch.int32, device="cuda")
+    q = torch.randn(B, Hkv * group, 1, D, generator=g, device="cuda", dtype=torch.float16)
+    kc = torch.randn(B, Hkv, Lmax, D, generator=g, device="cuda", dtype=torch.float16)
+    vc = torch.randn(B, Hkv, Lmax, D, generator=g, device="cuda", dtype=torch.float16)
+    out = torch.zeros_like(q)
+    kerns.flash_attn_decode(q, kc, vc, lens, out)
+    err = chunked = 0.0
+    for b in range(B):
+        n = int(lens[b])
+        s = (q[b].double().view(Hkv, group, D) @ kc[b].double().transpose(1, 2)) * (D ** -0.5 * 1.4426950408889634)
+        s[..., n:] = -float("inf")
+        v = vc[b].double()
+        p = torch.exp2(s - s.amax(-1, keepdim=True))
+        want = ((p / p.sum(-1, keepdim=True)) @ v).view(Hkv * group, 1, D)
+        tiles = s.view(Hkv, group, Lmax // 512, 8, 4, 16)             # chunk, tile of the warp, warp, key
+        ref = tiles.amax(-1).cummax(3).values.unsqueeze(-1)
+        w = torch.exp2(tiles - ref).nan_to_num(0.0)                  # (chunks beyond the sequence)
+        scale = torch.exp2(ref - s.amax(-1).view(Hkv, group, 1, 1, 1, 1))
+        num = (w.half().double() * scale).view(Hkv, group, Lmax) @ v
+        emu = (num / (w * scale).sum((2, 3, 4, 5)).unsqueeze(-1)).view(Hkv * group, 1, D).half().double()
+        err += float(((out[b].double() - want) ** 2).sum())
+        chunked += float(((emu - want) ** 2).sum())
+    assert err ** 0.5 <= 1.01 * chunked ** 0.5, (err / chunked) ** 0.5
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Hkv,group,D", [(1, 4, 128), (40, 9, 64)])
+def test_scores_that_fall_or_rise_along_the_sequence(kerns, dtype, Hkv, group, D):
+    """The reference maximum of a warp goes down by 2^4 per segment: scores that fall by more than that from segment to segment
+    (the sums are then those of the first keys), that rise, and that stay within a segment's reach.  Tolerance: every weight
+    and the result carry one 16-bit rounding, and scores of up to 1100 octaves some 2e-4 of a weight in 32 bits."""
+    B, L = 3, 6000
+    g = torch.Generator().manual_seed(D)
+    q = torch.zeros(B, Hkv * group, 1, D)
+    q[..., 0] = D ** 0.5
+    kc = torch.randn(B, Hkv, L, D, generator=g) * 0.1
+    at = torch.arange(L, dtype=torch.float32)
+    kc[0, :, :, 0] = -at / 8                 # 11.5 octaves per 64 keys, down
+    kc[1, :, :, 0] = (at - L) / 8            # and up
+    kc[2, :, :, 0] = -at / 400
+    vc = torch.randn(B, Hkv, L, D, generator=g) * 100
+    q, kc, vc = q.to(dtype), kc.to(dtype), vc.to(dtype)
+    lens = torch.tensor([L, L - 3, L - 7], dtype=torch.int32)
+    got = run_decode(kerns, q, kc, vc, lens).float().cpu()
+    want = O.attention_f64(q, kc, vc, lens=lens)
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    tol = (u + 3e-4) * O.attention_f64(q, kc, vc.abs(), lens=lens) + u * want.abs()
+    assert ((got - want).abs() <= tol).all(), float(((got - want).abs() / tol).max())
