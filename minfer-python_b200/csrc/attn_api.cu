@@ -149,22 +149,38 @@ int32_t default_chunk(int32_t batch, int32_t n_kv_heads, int32_t max_len) {
 bool decode_is_large(int64_t pairs, int64_t max_len, int64_t row_bytes) { return pairs * max_len * row_bytes * 2 > (int64_t{160} << 20); }
 
 // Blocks (one cluster) per (sequence, kv head) of a decode call, or 0: chunks, and a second kernel that merges them.
-// The lengths are on the device, so the rule knows the padded length only.
-//   A block costs about 4 us beside its keys (launch, the chain length -> keys -> scores, merge), and two fit an SM, four
-//   at head_dim 64.  While the caches hold little, a call is one such latency: as many blocks as one wave takes, no more.
-//   Measured (us, 1 / 2 / 4 / 8 / 16 blocks): 1 sequence, 8 kv heads, 777 keys, D=128 7.7 / 6.0 / 4.9 / 4.4 / 4.4; 8
-//   sequences of 513-640, D=64 6.8 / 6.6 / 6.1 / 5.8 / 11.5; 8 of 2000-4096, D=128 33 / 22.5 / 19.3 / 20.7 / 31; 32 of 300
-//   9.4 / 13.6 / 20 / 32 / 70.
-//   Large caches (worth 25 us of bandwidth and more) are taken in several waves, so that a batch of ragged lengths
-//   leaves no long tail (with the longest sequences first, see sequence_by_length): 64 sequences of 512-8192, 8 kv heads
-//   177 / 164 / 174 / 203; 24 of 100-6000 71 / 53.7 / 54.7 / 72; Q8_0, 64 of 512-8192 150 / 106 / 118 / 150.
-//   A handful of heads over a very long cache would leave most SMs without a block: chunks then.
+// The lengths are on the device, so the rule knows the padded length only; Q8_0 caches follow the 16-bit ones, so that both
+// split a sequence alike and their sums agree bit for bit.  Measured over 1085 shapes (1-1024 pairs of a sequence and a kv
+// head, 256-262144 keys, all of them visible or evenly spread from a sixteenth up) against chunks of 128-512 keys and a merging kernel;
+// all times us, back to back in a graph, D=128, groups of 4, 16-bit, unless said otherwise.
+//   A block costs some 3 us beside its keys, and two fit an SM (four at head_dim 64): as many blocks as one wave takes.
+//   1 / 2 / 4 / 8 / 16 blocks: 8 pairs of 4096 keys 28.8 / 16.8 / 10.4 / 7.7 / 6.9; 64 pairs of 512-8192 57 / 35 / 28 / 29 / 44.
+//   More than a wave only pays where a block still has many keys, and then mostly for ragged batches, whose tail it shortens
+//   (with the longest sequences first, see sequence_by_length): two waves from 256 KB of keys per block, 128 pairs of
+//   512-8192 51 (2 blocks) / 46 (4) / 55 (8); 512 pairs of 128-2048 46 (1) / 57 (2); three and a half from 512 KB, 512 pairs of
+//   512-8192 Q8_0 125 (1) / 109 (2) / 124 (4).
+//   A cluster of 16 wants eight free SMs of one processing cluster, so only some dozen of them run at a time.  Beyond
+//   that many pairs 8 blocks are better - 16 pairs of 1024 keys 5.5 (8) / 8.5 (16), 64 pairs of 8192 48 / 61 - unless the blocks
+//   are long and the batch may be ragged: 16 pairs of 512-8192 13.8 / 11.0, of 16384 27.6 / 33.0; 32 pairs of 2048-32768 at D=64 34 / 29.
+//   Few pairs of a very long cache keep 64 blocks or less busy that way.  Chunks / 16 blocks: 1 pair of 32768 30 / 19, of 65536
+//   58 / 35, of 131072 62 / 65, of 262144 72 / 122; 2 pairs of 32768 35 / 20, Q8_0 of 65536 39 / 49; 3 pairs Q8_0 of 65536 30 /
+//   48; 5 sequences of 8192-131072 Q8_0 51 / 94.  From 8 pairs on the two forms of cache part ways (8 pairs of 65536 67 / 48, Q8_0
+//   54 / 65), and the line stays where 16-bit caches want it.
 int decode_parts(int64_t batch, int64_t n_kv_heads, int64_t max_len, int64_t row_bytes) {
   const int64_t pairs = batch * n_kv_heads;
-  if (pairs <= 4 && max_len >= 32768) return 0;
-  const int64_t limit = decode_is_large(pairs, max_len, row_bytes) ? 1024 : (row_bytes == 128 ? 4 : 2) * 148;
+  if (max_len >= 32768 && pairs * max_len > 65536 && pairs <= (batch > 1 ? 6 : 4)) return 0;
+  const int64_t wave = (row_bytes == 128 ? 4 : 2) * 148;
   int parts = 1;
-  while (parts < 16 && pairs * parts * 2 <= limit && max_len >= 64 * parts * 2) parts *= 2;
+  while (parts < 16 && max_len >= 64 * parts * 2) {
+    const int next = parts * 2;
+    const int64_t block_bytes = max_len / next * row_bytes;  // of keys; as many of values
+    const int64_t limit = block_bytes >= (512 << 10) ? wave * 7 / 2 : block_bytes >= (256 << 10) ? wave * 2 : wave;
+    if (pairs * next > limit) break;
+    if (next == 16 && pairs > (row_bytes == 128 ? 24 : 12) &&
+        !(pairs <= 16 && block_bytes >= (128 << 10)) && !(pairs <= 32 && block_bytes >= (512 << 10)))
+      break;
+    parts = next;
+  }
   return parts;
 }
 

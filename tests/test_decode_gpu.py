@@ -178,9 +178,11 @@ def test_random_shapes_against_the_oracle(kerns, seed):
 
 @pytest.mark.parametrize("B,Hkv,group,D,Lmax,dtype", [
     (1, 1, 1, 64, 15, torch.float16), (1, 2, 16, 128, 1100, torch.bfloat16),   # one block; clusters of 16, two column tiles
-    (9, 2, 9, 64, 1024, torch.float16), (40, 2, 4, 128, 150, torch.float16),   # clusters of 8 and of 2
+    (9, 2, 9, 64, 1024, torch.float16), (40, 2, 4, 128, 150, torch.float16),   # clusters of 16 and of 2
+    (16, 1, 4, 128, 1100, torch.bfloat16), (10, 6, 3, 128, 700, torch.float16),     # clusters of 8 and of 4
     (150, 2, 8, 64, 300, torch.bfloat16),                                      # more pairs than one wave of blocks
-    (256, 1, 2, 128, 1300, torch.float16), (257, 1, 2, 128, 1300, torch.float16)])  # large, ordered by length and not
+    (256, 1, 2, 128, 1300, torch.float16), (257, 1, 2, 128, 1300, torch.float16),   # one block each, a batch that could be ranked and one that could not
+    (256, 1, 2, 128, 2048, torch.float16), (257, 1, 2, 128, 2048, torch.float16)])  # two waves, ordered by length and not
 def test_block_clusters_and_order_by_length(kerns, B, Hkv, group, D, Lmax, dtype):
     """Every cluster size and both orders, with lengths at the edges of the 16-key tiles and of the shares of a
     cluster's blocks (so that some blocks get nothing), empty sequences and equal lengths among them."""
@@ -229,7 +231,7 @@ def test_infinite_values_and_nan_scores(kerns, D, H, Hkv, Lmax, dtype):
     assert torch.count_nonzero(got[1:]) == 0
 
 
-@pytest.mark.parametrize("B,Hkv,Lmax", [(6, 8, 6912), (13, 8, 3264), (255, 1, 1300), (256, 1, 1300)])
+@pytest.mark.parametrize("B,Hkv,Lmax", [(6, 8, 8192), (13, 8, 4096), (255, 1, 2048), (256, 1, 2048)])
 def test_lengths_outside_the_cache_are_clamped_in_order_by_length(kerns, B, Hkv, Lmax):
     """Calls that take the longest sequences first, batches that are and are not multiples of four: a negative length is an
     empty sequence (zeros), one beyond the cache is max_len, and no sequence is lost - the bits of the same call with clamped lengths."""
@@ -309,3 +311,32 @@ def test_scores_that_fall_or_rise_along_the_sequence(kerns, dtype, Hkv, group, D
     u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     tol = (u + 3e-4) * O.attention_f64(q, kc, vc.abs(), lens=lens) + u * want.abs()
     assert ((got - want).abs() <= tol).all(), float(((got - want).abs() / tol).max())
+
+
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("B,Hkv,Lmax", [(1, 1, 32768), (1, 3, 32768), (5, 1, 32768), (1, 5, 32768), (16, 1, 8192), (1, 1, 65552)])
+def test_few_heads_over_a_long_cache(kerns, B, Hkv, Lmax, paged):
+    """Both sides of the lines between clusters of 16 blocks, of 8, and chunks merged by a second kernel, as the library
+    chooses them: full, ragged and empty sequences of a padded and of a paged cache."""
+    D, group = 128, 2
+    g = torch.Generator().manual_seed(B + Hkv)
+    q = torch.randn(B, Hkv * group, 1, D, generator=g).half()
+    kc = torch.randn(B, Hkv, Lmax, D, generator=g).half()
+    vc = torch.randn(B, Hkv, Lmax, D, generator=g).half()
+    lens = torch.tensor([Lmax, 0, Lmax // 2 + 3, 1, 700][:B] + [Lmax - 17 * i for i in range(5, B)], dtype=torch.int32)
+    want = O.attention_f64(q, kc, vc, lens=lens)
+    if not paged:
+        got = run_decode(kerns, q, kc, vc, lens)
+    else:
+        page = 16
+        per_seq = Lmax // page
+        table = torch.randperm(B * per_seq, generator=g).to(torch.int32).view(B, per_seq)
+        pools = []
+        for x in (kc, vc):
+            pool = torch.empty(B * per_seq, Hkv, page, D, dtype=x.dtype)
+            pool[table.long().flatten()] = x.view(B, Hkv, per_seq, page, D).transpose(1, 2).reshape(B * per_seq, Hkv, page, D)
+            pools.append(pool.cuda())
+        got = torch.full(q.shape, float("nan"), dtype=q.dtype, device="cuda")
+        kerns.flash_attn_decode_paged(q.cuda(), *pools, table.cuda(), lens.cuda(), got)
+    check_close(got, want, f"{B}x{Hkv} heads, {Lmax} keys")
+    assert torch.count_nonzero(got[lens == 0]) == 0
