@@ -15,6 +15,7 @@
 
 #include <array>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <utility>
 
@@ -39,35 +40,44 @@ void* current_stream() {
 // Device buffers this layer owns (the library itself allocates nothing): one status word per
 // device, one scratch buffer per (device, stream, purpose), grown on demand through torch's
 // allocator and kept for the life of the process.
+// g_mu guards the maps only and is never held while torch allocates: the allocator may want the interpreter's lock (it
+// records Python stacks when asked to), and the direct entry points come here with that lock held.
 std::mutex g_mu;
 std::map<int, Tensor*> g_status;
 std::map<std::array<int64_t, 3>, Tensor*> g_scratch;
 int g_max_ctas = 0;
 
 Tensor& status_word(const Tensor& like) {
-  std::lock_guard<std::mutex> lock(g_mu);
   const int dev = like.get_device_index();
-  auto it = g_status.find(dev);
-  if (it == g_status.end()) {
-    const int64_t n[1] = {4};
-    it = g_status.emplace(dev, new Tensor(torch::stable::new_zeros(like, {n, 1}, ScalarType::Int))).first;
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    auto it = g_status.find(dev);
+    if (it != g_status.end()) return *it->second;
   }
-  return *it->second;
+  const int64_t n[1] = {4};
+  auto mine = std::make_unique<Tensor>(torch::stable::new_zeros(like, {n, 1}, ScalarType::Int));
+  std::lock_guard<std::mutex> lock(g_mu);
+  Tensor*& kept = g_status[dev];  // another thread's, if it was quicker
+  if (kept == nullptr) kept = mine.release();
+  return *kept;
 }
 
 Tensor& scratch(const Tensor& like, void* stream, int64_t purpose, size_t bytes) {
-  std::lock_guard<std::mutex> lock(g_mu);
   const std::array<int64_t, 3> key = {like.get_device_index(), reinterpret_cast<int64_t>(stream), purpose};
-  auto it = g_scratch.find(key);
-  if (it == g_scratch.end() || static_cast<size_t>(it->second->numel()) < bytes) {
-    // powers of two, so that the outgrown buffers of a slowly growing series of calls add up to less than the last one
-    int64_t n[1] = {1 << 20};
-    while (static_cast<size_t>(n[0]) < bytes) n[0] *= 2;
-    Tensor* t = new Tensor(torch::stable::new_empty(like, {n, 1}, ScalarType::Byte));
-    if (it == g_scratch.end()) it = g_scratch.emplace(key, t).first;
-    else it->second = t;  // the old buffer stays alive: launches in flight may still use it
+  auto fits = [bytes](const Tensor* t) { return t != nullptr && static_cast<size_t>(t->numel()) >= bytes; };
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    auto it = g_scratch.find(key);
+    if (it != g_scratch.end() && fits(it->second)) return *it->second;
   }
-  return *it->second;
+  // powers of two, so that the outgrown buffers of a slowly growing series of calls add up to less than the last one
+  int64_t n[1] = {1 << 20};
+  while (static_cast<size_t>(n[0]) < bytes) n[0] *= 2;
+  auto mine = std::make_unique<Tensor>(torch::stable::new_empty(like, {n, 1}, ScalarType::Byte));
+  std::lock_guard<std::mutex> lock(g_mu);
+  Tensor*& kept = g_scratch[key];
+  if (!fits(kept)) kept = mine.release();  // an outgrown buffer stays alive: launches in flight may still use it
+  return *kept;
 }
 
 struct StableEnv {

@@ -157,3 +157,46 @@ def test_direct_entry_points_leave_everything_unusual_to_the_dispatcher(kerns):
     out2 = torch.zeros_like(out)
     torch.compile(lambda o: kerns.flash_attn_decode(q, k, v, lens, o), fullgraph=True, backend="eager")(out2)
     assert torch.equal(out, out2)
+
+
+_TWO_ROUTES = """
+import sys, threading
+sys.path.insert(0, sys.argv[1])
+import torch
+from minfer.kernels.torch_ext import ops
+torch.cuda.memory._record_memory_history(context="all", stacks="python")
+q = torch.randn(1, 4, 1, 64, device="cuda").half()
+k = torch.randn(1, 2, 64, 64, device="cuda").half()
+lens = torch.full((1,), 64, dtype=torch.int32, device="cuda")
+outs = [torch.zeros_like(q) for _ in range(2)]
+streams = [torch.cuda.Stream() for _ in range(32)]
+torch.cuda.synchronize()
+done = threading.Event()
+
+def dispatched():      # a new stream each time: a scratch buffer is allocated, and the allocator records this stack
+    for s in streams[2:]:
+        with torch.cuda.stream(s):
+            torch.ops.minfer.flash_attn_decode.default(q, k, k, lens, outs[0])
+    done.set()
+
+def direct():          # two streams in turn: the buffers are looked up in every call
+    while not done.is_set():
+        for s in streams[:2]:
+            with torch.cuda.stream(s):
+                assert ops._direct.flash_attn_decode(q, k, k, lens, outs[1])
+            s.synchronize()
+
+threads = [threading.Thread(target=f) for f in (direct, dispatched)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+torch.cuda.synchronize()
+assert torch.equal(*outs)
+print("both routes ended")
+"""
+
+
+def test_both_routes_at_once_while_the_allocator_records_python_stacks():
+    """The direct route comes to the buffers' lock with the interpreter's lock held, and the allocator wants the interpreter's
+    lock: no thread may allocate under the former.  (In a process of its own, which ends by the limit if two threads wait for each other.)"""
+    r = subprocess.run([sys.executable, "-c", _TWO_ROUTES, PKG_ROOT], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and "both routes ended" in r.stdout, r.stderr[-2000:]
