@@ -35,7 +35,7 @@ struct AttnOps {
   static int device_of(const T& t) { return Env::device_of(t); }
 
   // Scratch of a dense-mask call: with the tiles' bits (an eighth of the mask's bytes) while that is no more than 256 MB,
-  // as for masks up to 2 GB; beyond, the tile classes alone.
+  // as for masks up to 2 GB, and the device has room for it; otherwise the tile classes alone.
   static size_t mask_workspace_bytes(int32_t batch, int32_t seq_q, int32_t seq_k) {
     const size_t with_bits = minfer_attn_prefill_workspace_bytes_bits(batch, seq_q, seq_k);
     return with_bits <= (size_t{256} << 20) ? with_bits : minfer_attn_prefill_workspace_bytes(batch, seq_q, seq_k);
@@ -104,8 +104,9 @@ struct AttnOps {
     p.causal = causal ? 1 : 0;
     p.max_ctas = Env::max_ctas();
     void* stream = Env::stream(q);
-    const size_t need = mask != nullptr ? mask_workspace_bytes(p.batch, p.seq_q, p.seq_k) : 16;
-    const Scratch ws = Env::scratch(q, stream, /*purpose=*/0, need);
+    const size_t least = mask != nullptr ? minfer_attn_prefill_workspace_bytes(p.batch, p.seq_q, p.seq_k) : 16;
+    const size_t want = mask != nullptr ? mask_workspace_bytes(p.batch, p.seq_q, p.seq_k) : least;
+    const Scratch ws = Env::scratch(q, stream, /*purpose=*/0, want, least);
     p.workspace = ws.ptr;
     p.workspace_bytes = ws.bytes;
     check_rc(Env::call(minfer_attn_prefill, &p, stream), "minfer_attn_prefill");
@@ -146,7 +147,7 @@ struct AttnOps {
     for (int i = 0; i < 3; ++i) p.kv_stride[i] = kc.stride(i);
     void* stream = Env::stream(q);
     const size_t need = minfer_attn_decode_workspace_bytes(p.batch, p.n_heads, p.max_len, p.head_dim, 0);
-    const Scratch ws = Env::scratch(q, stream, /*purpose=*/1, need);
+    const Scratch ws = Env::scratch(q, stream, /*purpose=*/1, need, need);
     p.workspace = ws.ptr;
     p.workspace_bytes = ws.bytes;
     check_rc(Env::call(minfer_attn_decode, &p, stream), "minfer_attn_decode");

@@ -10,7 +10,8 @@
 namespace minfer {
 
 int32_t* binding_status(void* like);                                              // the device's status word
-Scratch binding_scratch(void* like, void* stream, int64_t purpose, size_t bytes);  // never moves while the process lives
+// `want` bytes where the device has them, `least` in any case; never moves while the process lives
+Scratch binding_scratch(void* like, void* stream, int64_t purpose, size_t want, size_t least);
 int binding_max_ctas();
 
 }  // namespace minfer

@@ -34,13 +34,13 @@ struct DirectEnv {
     if (known[dev] == nullptr) known[dev] = binding_status(const_cast<Tensor*>(&like));
     return known[dev];
   }
-  static Scratch scratch(const Tensor& like, void* stream, int64_t purpose, size_t bytes) {
+  static Scratch scratch(const Tensor& like, void* stream, int64_t purpose, size_t want, size_t least) {
     // the latest buffer of each purpose: buffers are kept for the life of the process, so a remembered one stays valid
     struct Entry { int dev; void* stream; Scratch s; };
     thread_local std::array<Entry, 2> last{Entry{-1, nullptr, {}}, Entry{-1, nullptr, {}}};
     Entry& e = last[purpose & 1];
-    if (e.dev != like.get_device() || e.stream != stream || e.s.bytes < bytes)
-      e = Entry{like.get_device(), stream, binding_scratch(const_cast<Tensor*>(&like), stream, purpose, bytes)};
+    if (e.dev != like.get_device() || e.stream != stream || e.s.bytes < want)
+      e = Entry{like.get_device(), stream, binding_scratch(const_cast<Tensor*>(&like), stream, purpose, want, least)};
     return e.s;
   }
   static int max_ctas() { return binding_max_ctas(); }

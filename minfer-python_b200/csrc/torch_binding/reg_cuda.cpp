@@ -14,6 +14,7 @@
 #include <torch/csrc/stable/c/shim.h>
 
 #include <array>
+#include <exception>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -44,7 +45,12 @@ void* current_stream() {
 // records Python stacks when asked to), and the direct entry points come here with that lock held.
 std::mutex g_mu;
 std::map<int, Tensor*> g_status;
-std::map<std::array<int64_t, 3>, Tensor*> g_scratch;
+struct ScratchSlot {
+  Tensor* buffer = nullptr;
+  size_t refused = 0;  // the smallest size beyond `least` that could not be had, 0: none
+  int passed_over = 0;  // calls since then that did without
+};
+std::map<std::array<int64_t, 3>, ScratchSlot> g_scratch;
 int g_max_ctas = 0;
 
 Tensor& status_word(const Tensor& like) {
@@ -62,22 +68,45 @@ Tensor& status_word(const Tensor& like) {
   return *kept;
 }
 
-Tensor& scratch(const Tensor& like, void* stream, int64_t purpose, size_t bytes) {
-  const std::array<int64_t, 3> key = {like.get_device_index(), reinterpret_cast<int64_t>(stream), purpose};
-  auto fits = [bytes](const Tensor* t) { return t != nullptr && static_cast<size_t>(t->numel()) >= bytes; };
-  {
-    std::lock_guard<std::mutex> lock(g_mu);
-    auto it = g_scratch.find(key);
-    if (it != g_scratch.end() && fits(it->second)) return *it->second;
-  }
+bool fits(const ScratchSlot& slot, size_t bytes) {
+  return slot.buffer != nullptr && static_cast<size_t>(slot.buffer->numel()) >= bytes;
+}
+
+Tensor& grow_scratch(const Tensor& like, const std::array<int64_t, 3>& key, size_t bytes) {
   // powers of two, so that the outgrown buffers of a slowly growing series of calls add up to less than the last one
   int64_t n[1] = {1 << 20};
   while (static_cast<size_t>(n[0]) < bytes) n[0] *= 2;
   auto mine = std::make_unique<Tensor>(torch::stable::new_empty(like, {n, 1}, ScalarType::Byte));
   std::lock_guard<std::mutex> lock(g_mu);
-  Tensor*& kept = g_scratch[key];
-  if (!fits(kept)) kept = mine.release();  // an outgrown buffer stays alive: launches in flight may still use it
-  return *kept;
+  ScratchSlot& slot = g_scratch[key];
+  if (!fits(slot, bytes)) slot.buffer = mine.release();  // an outgrown buffer stays alive: launches in flight may still use it
+  return *slot.buffer;
+}
+
+// At least `least` bytes, and `want` where the device has them.  A refused allocation is costly (torch gives its cached
+// blocks back and tries again), so on a full device the larger size is asked for once in 256 calls only.
+Tensor& scratch(const Tensor& like, void* stream, int64_t purpose, size_t want, size_t least) {
+  const std::array<int64_t, 3> key = {like.get_device_index(), reinterpret_cast<int64_t>(stream), purpose};
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    ScratchSlot& slot = g_scratch[key];
+    if (fits(slot, want)) return *slot.buffer;
+    if (least < want && slot.refused != 0 && want >= slot.refused && ++slot.passed_over % 256 != 0) {
+      if (fits(slot, least)) return *slot.buffer;
+      want = least;
+    }
+  }
+  if (least < want) {
+    try {
+      return grow_scratch(like, key, want);
+    } catch (const std::exception&) {
+      std::lock_guard<std::mutex> lock(g_mu);
+      ScratchSlot& slot = g_scratch[key];
+      if (slot.refused == 0 || want < slot.refused) slot.refused = want;
+      if (fits(slot, least)) return *slot.buffer;
+    }
+  }
+  return grow_scratch(like, key, least);
 }
 
 struct StableEnv {
@@ -85,8 +114,8 @@ struct StableEnv {
   static int device_of(const Tensor& t) { return t.get_device_index(); }
   static void* stream(const Tensor&) { return current_stream(); }
   static int32_t* status(const Tensor& like) { return static_cast<int32_t*>(status_word(like).mutable_data_ptr()); }
-  static Scratch scratch(const Tensor& like, void* stream, int64_t purpose, size_t bytes) {
-    Tensor& t = minfer::scratch(like, stream, purpose, bytes);
+  static Scratch scratch(const Tensor& like, void* stream, int64_t purpose, size_t want, size_t least) {
+    Tensor& t = minfer::scratch(like, stream, purpose, want, least);
     return {t.mutable_data_ptr(), static_cast<size_t>(t.numel())};
   }
   static int max_ctas() { return g_max_ctas; }
@@ -105,8 +134,8 @@ Tensor borrowed(void* at_tensor) {  // a stable tensor sharing the at::Tensor be
 
 // the buffers, for the direct entry points (buffers.h)
 int32_t* binding_status(void* like) { return StableEnv::status(borrowed(like)); }
-Scratch binding_scratch(void* like, void* stream, int64_t purpose, size_t bytes) {
-  return StableEnv::scratch(borrowed(like), stream, purpose, bytes);
+Scratch binding_scratch(void* like, void* stream, int64_t purpose, size_t want, size_t least) {
+  return StableEnv::scratch(borrowed(like), stream, purpose, want, least);
 }
 int binding_max_ctas() { return g_max_ctas; }
 

@@ -181,12 +181,17 @@ def _prefill(q, k, v, mask, out, causal: bool, peer_out=()) -> None:
     p.flags = 0
     p.max_ctas = _max_ctas
     # mask tile classes (dense mask) or the persistent kernel's work-item counter (causal)
-    need = 16
-    if mask is not None:   # with the mask tiles' bits while they are no more than 256 MB
-        need = _lib.lib.minfer_attn_prefill_workspace_bytes_bits(p.batch, p.seq_q, p.seq_k)
-        if need > 256 << 20:
-            need = _lib.lib.minfer_attn_prefill_workspace_bytes(p.batch, p.seq_q, p.seq_k)
-    ws = _workspace_for(q.device, need, _mask_workspace, torch.cuda.current_stream(q.device).cuda_stream)
+    least = want = 16
+    if mask is not None:   # with the mask tiles' bits while they are no more than 256 MB and the device has room for them
+        least = _lib.lib.minfer_attn_prefill_workspace_bytes(p.batch, p.seq_q, p.seq_k)
+        want = _lib.lib.minfer_attn_prefill_workspace_bytes_bits(p.batch, p.seq_q, p.seq_k)
+        if want > 256 << 20:
+            want = least
+    stream = torch.cuda.current_stream(q.device).cuda_stream
+    try:
+        ws = _workspace_for(q.device, want, _mask_workspace, stream)
+    except torch.OutOfMemoryError:
+        ws = _workspace_for(q.device, least, _mask_workspace, stream)
     p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     with torch.cuda.device(q.device):
         stream = torch.cuda.current_stream().cuda_stream

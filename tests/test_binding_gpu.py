@@ -200,3 +200,52 @@ def test_both_routes_at_once_while_the_allocator_records_python_stacks():
     lock: no thread may allocate under the former.  (In a process of its own, which ends by the limit if two threads wait for each other.)"""
     r = subprocess.run([sys.executable, "-c", _TWO_ROUTES, PKG_ROOT], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and "both routes ended" in r.stdout, r.stderr[-2000:]
+
+
+_FULL_DEVICE = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+from minfer.kernels import KernelBackend
+from minfer.kernels.torch_ext import ops
+kerns = KernelBackend("torch_ext")
+F16 = (1, 1, 2)
+L = 6000                                       # the tiles' bits: 4.5 MB, their classes: 2 KB
+g = torch.Generator(device="cuda").manual_seed(5)
+q, k, v = (torch.randn(1, h, L, 64, generator=g, device="cuda").half() for h in (2, 1, 1))
+mask = torch.rand(1, 1, L, L, generator=g, device="cuda") < 0.5
+outs = [torch.zeros_like(q) for _ in range(3)]
+stream = torch.cuda.Stream()
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+total = torch.cuda.get_device_properties(0).total_memory
+torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (4 << 20)) / total)    # 4 MB left
+try:
+    with torch.cuda.stream(stream):            # (the allocator keeps a pool per stream)
+        torch.empty(8 << 20, dtype=torch.uint8, device="cuda")
+    raise SystemExit("the device is not full")
+except torch.OutOfMemoryError:
+    pass
+calls = [lambda o: kerns.flash_attn(*F16, q, k, v, mask, o), lambda o: torch.ops.minfer.flash_attn.default(*F16, q, k, v, mask, o)]
+with torch.cuda.stream(stream):
+    for call, out in zip(calls, outs):
+        for _ in range(3):
+            call(out)
+torch.cuda.synchronize()
+torch.cuda.set_per_process_memory_fraction(1.0)
+with torch.cuda.stream(stream):
+    for _ in range(260):                       # room again: the larger scratch is asked for within 256 calls
+        kerns.flash_attn(*F16, q, k, v, mask, outs[2])
+torch.cuda.synchronize()
+assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+assert torch.isfinite(outs[0]).all() and outs[0].abs().sum() > 0
+print("served")
+"""
+
+
+@pytest.mark.parametrize("binding", ["auto", "ctypes"])
+def test_dense_mask_on_a_full_device(binding):
+    """The scratch for the mask tiles' bits cannot be had: the call is served with the tile classes alone, with the same bits."""
+    r = subprocess.run([sys.executable, "-c", _FULL_DEVICE, PKG_ROOT], capture_output=True, text=True, timeout=240,
+                       env={**os.environ, "MINFER_ATTN_BINDING": binding})
+    assert r.returncode == 0 and "served" in r.stdout, r.stdout + r.stderr[-2000:]
