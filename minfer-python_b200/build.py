@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -98,8 +99,15 @@ def direct_path() -> str:
     return os.path.join(OUT_DIR, "_direct" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
-def build_direct(force: bool = False, verbose: bool = False) -> str:
-    """Compile `minfer.kernels.torch_ext._direct` against torch's C++ headers and link it to _C and the library."""
+def direct_stamp_path() -> str:
+    """Which torch the present _direct was compiled against."""
+    return os.path.join(HERE, "build", "_direct.torch")
+
+
+def build_direct(force: bool = False, verbose: bool = False) -> str | None:
+    """Compile `minfer.kernels.torch_ext._direct` against torch's C++ headers and link it to _C and the library.
+    Everything works without it, so where it cannot be compiled (no headers of Python, torch or the CUDA runtime) there is a
+    warning and no file.  Unlike _C it is tied to the torch it was compiled against: another one makes it stale."""
     import sysconfig
 
     import torch
@@ -107,18 +115,33 @@ def build_direct(force: bool = False, verbose: bool = False) -> str:
     src = os.path.join(CSRC, DIRECT_SOURCE)
     newest = max(os.path.getmtime(f) for f in [src] + [os.path.join(CSRC, f) for f in BINDING_HEADERS] +
                  [os.path.join(INCLUDE, "minfer_attn.h"), binding_path()])
-    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
+    stamp = direct_stamp_path()
+    other_torch = False
+    if os.path.exists(stamp):
+        with open(stamp) as f:
+            other_torch = f.read() != torch.__version__
+    if not force and not other_torch and os.path.exists(out) and os.path.getmtime(out) >= newest:
         return out
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_find_nvcc()))
     cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I", os.path.join(tdir, "include"), "-I", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
-           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include"), src, "-o", out,
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include"),
+           f'-DMINFER_TORCH_VERSION="{torch.__version__}"', src, "-o", out,
            "-L", OUT_DIR, "-l:" + BINDING_NAME, "-l:" + LIB_NAME, "-Wl,-rpath,$ORIGIN",
            "-L", os.path.join(tdir, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     if verbose:
         print(" ".join(cmd), flush=True)
-    subprocess.run(cmd, check=True)
+    try:
+        subprocess.run(cmd, check=True)
+    except (OSError, subprocess.CalledProcessError) as e:
+        if os.path.exists(out):
+            os.remove(out)  # of other sources
+        warnings.warn(f"{os.path.basename(out)} could not be compiled ({e}): every call goes through torch's dispatcher")
+        return None
+    os.makedirs(os.path.dirname(stamp), exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(torch.__version__)
     return out
 
 

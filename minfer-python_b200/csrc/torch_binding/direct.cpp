@@ -190,4 +190,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_direct", "attention ops without t
 }  // namespace
 }  // namespace minfer
 
-PyMODINIT_FUNC PyInit__direct(void) { return PyModule_Create(&minfer::module); }
+// The tensors are read by the layout of the torch that this file was compiled against: ops.py asks which one that was.
+PyMODINIT_FUNC PyInit__direct(void) {
+  PyObject* m = PyModule_Create(&minfer::module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", MINFER_TORCH_VERSION) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

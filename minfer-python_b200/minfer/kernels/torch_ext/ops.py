@@ -89,12 +89,16 @@ if _binding_choice != "ctypes":
 BINDING = "stable" if _C is not None else "ctypes"
 # entry points that skip the dispatcher (csrc/torch_binding/direct.cpp): each returns whether it served the call, which
 # it does for plain CUDA tensors on the current device with nothing on the thread that wants to see the op
-_direct = None
-if _C is not None and _binding_choice == "auto":
+def _load_direct():
     try:
         from . import _direct
     except ImportError:
-        _direct = None
+        return None
+    # it reads tensors in place, by the layout of the torch it was compiled against
+    return _direct if getattr(_direct, "torch_version", None) == torch.__version__ else None
+
+
+_direct = _load_direct() if _C is not None and _binding_choice == "auto" else None
 _is_compiling = torch.compiler.is_compiling  # a tracer has to meet the op itself
 # ops whose CUDA implementation lives in the extension
 _IN_EXTENSION = tuple(_DEFS) if _C is not None else ()

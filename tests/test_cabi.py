@@ -3,10 +3,11 @@ rejects bad arguments before touching a device."""
 import ctypes
 import os
 import re
+import sys
 
 import pytest
 
-from conftest import ROOT
+from conftest import PKG_ROOT, ROOT
 
 
 def declared_symbols():
@@ -157,3 +158,50 @@ def test_refs_rope_matches_the_oracle_restatement():
     for rot in (64, 32):
         assert torch.allclose(refs.il_rope(x, rot, 7, 10000.0).float(), O.il_rope_reference(x, rot, 7, 10000.0).float(), atol=2e-3)
         assert torch.allclose(refs.neox_rope(x, rot, 7, 10000.0).float(), O.neox_rope_reference(x, rot, 7, 10000.0).float(), atol=2e-3)
+
+
+def _native_build():
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("minfer_b200_build_under_test", os.path.join(PKG_ROOT, "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+def test_build_goes_on_without_the_direct_entry_points(monkeypatch, tmp_path):
+    """No compiler that can build `_direct` (missing headers): build() warns, leaves no file of other sources and returns the library."""
+    import subprocess
+    mod = _native_build()
+    stale = tmp_path / "_direct.so"
+    stale.write_bytes(b"of other sources")
+    run = subprocess.run
+
+    def fails(cmd, **kw):
+        if any(str(a).endswith("direct.cpp") for a in cmd):
+            raise subprocess.CalledProcessError(1, cmd)
+        return run(cmd, **kw)
+
+    monkeypatch.setattr(mod, "direct_path", lambda: str(stale))
+    monkeypatch.setattr(mod, "direct_stamp_path", lambda: str(tmp_path / "stamp"))
+    (tmp_path / "stamp").write_text("0.0")     # compiled against another torch
+    monkeypatch.setattr(mod.subprocess, "run", fails)
+    with pytest.warns(UserWarning, match="dispatcher"):
+        assert os.path.samefile(mod.build(), mod.lib_path())
+    assert not stale.exists()
+
+
+def test_direct_entry_points_of_another_torch_are_not_used(monkeypatch):
+    import types
+
+    import torch
+    import minfer.kernels.torch_ext as pkg
+    from minfer.kernels.torch_ext import ops
+    for version, used in ((torch.__version__, True), ("2.0.0", False), (None, False)):
+        fake = types.ModuleType("minfer.kernels.torch_ext._direct")
+        if version is not None:
+            fake.torch_version = version
+        monkeypatch.setattr(pkg, "_direct", fake, raising=False)
+        monkeypatch.setitem(sys.modules, fake.__name__, fake)
+        assert (ops._load_direct() is fake) == used
+    monkeypatch.undo()
+    assert ops._direct is None or ops._direct.torch_version == torch.__version__
