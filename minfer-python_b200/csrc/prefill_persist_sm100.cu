@@ -1099,8 +1099,10 @@ cudaError_t launch_persist_one(const CUtensorMap& tq, const CUtensorMap& tk, con
   // (43.9 with the memset left in).  Longer calls are launched in the
   // ordinary way: nothing to gain, and CTAs that take the SMs in the order in which the kernel in front leaves
   // them share less in L2 (dense mask, window 256, L=4096: 319 -> 325 us; 1000 queries on 16000 keys 240 -> 242 us).
+  // So is a call whose grid the caller has limited: the SMs that it leaves free are for another stream's kernel, and the
+  // CTAs of the call behind it would take them to wait there.
   const int n_kt = (a.seq_k + kTileN - 1) / kTileN;
-  a.programmatic = ((n_items + ctas - 1) / ctas) * n_kt <= 64 ? 1 : 0;
+  a.programmatic = (ctas == sms && ((n_items + ctas - 1) / ctas) * n_kt <= 64) ? 1 : 0;
   if (a.counter != nullptr && a.cls == nullptr) {
     if (a.programmatic) {
       LaunchAttrs zt(stream);

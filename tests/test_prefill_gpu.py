@@ -554,3 +554,37 @@ def test_calls_of_one_stream_in_a_row(kerns, L, H):
         for a, b in zip(run(False), want):
             assert torch.equal(a, b)
     check_close(want[0], O.attention_f64(*(x.cpu() for x in sets[0]), mask=masks[0].cpu()), f"L={L} H={H}")
+
+
+def test_limited_grids_leave_their_sms_to_other_streams(kerns):
+    """A call under a grid limit is not set up beside the call in front of it (on the SMs that the limit keeps free): it has no
+    programmatic edge in a captured graph, while short calls without a limit have them."""
+    from cuda.bindings import runtime as rt
+    from minfer.kernels.torch_ext import ops
+    q, k, v = (x.cuda() for x in seeded_qkv(3, 2, 8, 2, 300, 300, 64, torch.float16))
+    start = torch.zeros(2, dtype=torch.int32, device="cuda")
+    tok = [torch.randn(2, 1, h, 64, device="cuda").half() for h in (8, 2, 2)]
+    outs = [torch.zeros_like(q) for _ in range(3)]
+
+    def calls():
+        kerns.rope_kv_append(64, 10000.0, 0, *tok, k, v, start)
+        for out in outs:
+            kerns.flash_attn_causal(q, k, v, out)
+
+    def programmatic_edges(limit):
+        with ops.prefill_cta_limit(limit):
+            calls()
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph(keep_graph=True)
+            with torch.cuda.graph(graph):
+                calls()
+        raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+        err, *_, n = rt.cudaGraphGetEdges_v2(raw, 0)
+        assert err == rt.cudaError_t.cudaSuccess and n > 0
+        err, _, _, data, n = rt.cudaGraphGetEdges_v2(raw, n)
+        assert err == rt.cudaError_t.cudaSuccess
+        return sum(int(d.type) == int(rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for d in data)
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert programmatic_edges(0) > 0 and programmatic_edges(sms) > 0
+    assert programmatic_edges(4) == 0 and programmatic_edges(sms - 8) == 0
