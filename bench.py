@@ -672,9 +672,10 @@ print(json.dumps(res))
 
 def host_overhead_record():
     """CPU-side cost of one op call (microseconds, 10 k calls on tiny shapes so that the device never back-pressures
-    the host), for the torch-extension binding and for the ctypes binding, each in a process of its own."""
+    the host): what an ordinary call takes (the direct entry points), the torch extension through the dispatcher, and the
+    ctypes binding, each in a process of its own."""
     out = {}
-    for binding in ("stable", "ctypes"):
+    for binding in ("auto", "stable", "ctypes"):
         env = dict(os.environ, MINFER_ATTN_BINDING=binding)
         script = HOST_OVERHEAD_SCRIPT.format(pkg=os.path.join(ROOT, "minfer-python_b200"))
         try:
