@@ -21,16 +21,17 @@
 // Precision: the weights are rounded to 16 bits relative to the reference maximum, so a weight of exactly 1 - the largest
 // key's so far - costs nothing, and that is worth more the fewer keys share a maximum.  Therefore the maximum is exact
 // within a segment (letting it lag by up to 2^8, as the prefill kernel does, gives 2.9e-4 of the output at float16 against
-// 64 bits), and every chunk / 64 tiles - as many as a warp has of a chunk in the form with chunks - the reference is
-// lowered by 2^4, so that the next segment's largest keys set it again.  64 sequences of 512-8192 (float16 / bfloat16): 2.57e-4 / 2.06e-3;
-// one maximum for all keys of a warp 2.65e-4 / 2.12e-3; chunks of 512 keys 2.59e-4 / 2.07e-3.  What it costs (us, with / without): 16-bit 165.6 /
-// 165.2, Q8_0 116 / 109, one sequence of 16384, 8 kv heads 15.5 / 15.1.  (A second product with the rounding errors of
-// the weights gives 2.07e-4, but an infinite value times an error of 0 is NaN.)
+// 64 bits), and every chunk / 64 tiles - as many as a warp has of a chunk in the form with chunks - the reference may
+// fall by 2^4, so that the next segment's largest keys set it again.  64 sequences of 512-8192, float16 / bfloat16:
+// 2.57e-4 / 2.06e-3; one maximum for all keys of a warp 2.65e-4 / 2.12e-3; chunks of 512 keys 2.59e-4 / 2.07e-3.  What it
+// costs (us, with / without): those 64 sequences 165.6 / 165.2, Q8_0 115 / 109.7; one of 8192 keys, 8 kv heads, Q8_0 13.6 / 13.3;
+// 8 of 48-777 6.9 / 6.8.  (As a block of its own in front of the tile, which scaled O and the sums: 116, 14.0, 7.1.  A second
+// product with the rounding errors of the weights gives 2.07e-4, but an infinite value times an error of 0 is NaN.)
 //
 // The blocks of one (sequence, kv head) form a cluster: they share the sequence's actual tiles evenly - a padded
 // cache has no empty blocks - and each pushes its partial output into the shared memory of the block that finishes
-// that slice of the result, so one launch does the whole call and no partial result touches memory (split-KV with a
-// second, merging kernel took 4.2 + 2.8 us where this takes 4.7 together, and 6 us behind the batch-64 call).  Calls
+// that slice of the result, so one launch does the whole call and no partial result touches memory (one
+// sequence of 777 keys, 8 kv heads: 4.3 us, with chunks and a merging kernel 6.8).  Calls
 // with an explicit chunk, or a handful of heads over a very long cache (see decode_parts in attn_api.cu), write partials to the workspace
 // instead, merged by decode_combine_kernel.
 //
@@ -379,28 +380,6 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
     __syncwarp();
     issue_tile(i + kSt - 1);
 
-    // ---- a new segment: the reference maximum is lowered (O and the sums scaled by the same power of two, exactly), so that
-    // this segment's largest scores move it; not while a sum is large, so that a long run of falling scores cannot overflow ----
-    if ((i & seg_mask) == 0 && i > 0) {
-      bool room = true;
-#pragma unroll
-      for (int n = 0; n < NT; ++n) room = room && fmaxf(l_run[n][0], l_run[n][1]) < 512.f;
-      if (__all_sync(0xFFFFFFFFu, room)) {
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            m_ref[n][h] -= 4.f;
-            l_run[n][h] *= 16.f;
-          }
-#pragma unroll
-          for (int m = 0; m < D / 16; ++m)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) oacc[n][m][e] *= 16.f;
-        }
-      }
-    }
-
     const int key0 = c0 + (warp + i * kWarps) * kTileKeys;
     // ---- S^T[16 keys x 8 heads] = K Q^T ----
     // (two accumulators: half the length of the chain of dependent MMAs)
@@ -450,11 +429,13 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
       for (int e = 0; e < 4; ++e) s[n][e] += s2[n][e];
 
     // ---- online softmax over the keys: x = s * scale - maximum so far; a tile in which no score exceeds it needs no
-    // reduction over the lanes ----
+    // reduction over the lanes.  The first tile of a segment lets the reference fall (by up to 2^4, to its own maximum);
+    // not while a sum is large, so that a long run of falling scores cannot overflow. ----
     const bool partial = key0 + kTileKeys > c1;
     const bool dead0 = partial && key0 + g0 >= c1, dead1 = partial && key0 + g0 + 8 >= c1;
     float x[NT][4];
-    bool move = false;
+    const bool fresh = (i & seg_mask) == 0;
+    bool move = fresh;
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
 #pragma unroll
@@ -465,6 +446,10 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
       move |= fmaxf(fmaxf(x[n][0], x[n][1]), fmaxf(x[n][2], x[n][3])) > 0.f;
     }
     if (__any_sync(0xFFFFFFFFu, move)) {
+      bool room = fresh;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) room = room && fmaxf(l_run[n][0], l_run[n][1]) < 512.f;
+      const float drop = __all_sync(0xFFFFFFFFu, room) ? 4.f : 0.f;
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
         float alpha[2];
@@ -474,7 +459,7 @@ __global__ void __launch_bounds__(kWarps * 32, (Q8 && NT == 1) ? MINFER_ATTN_Q8_
           mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 4));
           mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 8));
           mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 16));
-          const float m_new = fmaxf(m_ref[n][h], mx);  // finite: every tile holds at least one live key
+          const float m_new = fmaxf(m_ref[n][h] - drop, mx);  // finite: every tile holds at least one live key
           alpha[h] = ex2_approx(m_ref[n][h] - m_new);  // first tile: exp2(-inf) = 0
           m_ref[n][h] = m_new;
           l_run[n][h] *= alpha[h];
