@@ -31,8 +31,8 @@
 // The blocks of one (sequence, kv head) form a cluster: they share the sequence's actual tiles evenly - a padded
 // cache has no empty blocks - and each pushes its partial output into the shared memory of the block that finishes
 // that slice of the result, so one launch does the whole call and no partial result touches memory (one
-// sequence of 777 keys, 8 kv heads: 4.3 us, with chunks and a merging kernel 6.8).  Calls
-// with an explicit chunk, or a handful of heads over a very long cache (see decode_parts in attn_api.cu), write partials to the workspace
+// sequence of 1024 keys, 8 kv heads: 4.6 us, with chunks and a merging kernel 6.9).  Calls with an explicit chunk, or a
+// handful of heads over a very long cache (see decode_parts in attn_api.cu), write partials to the workspace
 // instead, merged by decode_combine_kernel.
 //
 // Q8 = true: the caches hold GGML Q8_0 blocks (32 int8 + one fp16 scale, 34 bytes;
